@@ -533,13 +533,14 @@ int volume_args(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, Project
         int r = ensure_cells(ctx, v);
         if (r)
             return r;
-        mode = Mode::Cells;
+        mode = s->ray_sampling <= kSegmentMaxSampling ? Mode::Segments : Mode::Cells;
         a.cells = v.cells;
         const int n[3] = { (int)d.n[0], (int)d.n[1], (int)d.n[2] };
         const CellLayout L = cell_layout(n);
         a.csy = L.sy;
         a.csz = L.sz;
         a.cmax = L.max_index;
+        a.coffset = L.offset;
     }
     a.sy = a.ext[0];
     a.sz = a.ext[0] * a.ext[1];
@@ -970,7 +971,7 @@ int prepare_batch(ctlcu_ctx* ctx, const ctlcu_request* requests, uint32_t n, con
         int r = volume_args(ctx, *find_volume(ctx, q.volume), &eff, br.a, mode, dtype);
         if (r)
             return r;
-        if (mode != Mode::Cells && mode != Mode::Pairs)
+        if (mode != Mode::Cells && mode != Mode::Segments && mode != Mode::Pairs)
             return fail(ctx, CTLCU_ERR_INVALID_ARGUMENT, "request %u does not take the cell kernel", i);
         bp.mode = mode;
         job_args(br.a, &eff, q.n_views, q.n_modules, q.channels, q.rows);

@@ -19,7 +19,10 @@ constexpr int kPad = 2;
 
 // Register budgets of the sample loops (measured best; see the launch shapes below).
 #ifndef CTLCU_CELL_MAXREG
-#define CTLCU_CELL_MAXREG 48  // cell and pair loops: 5 blocks of 256 threads per SM
+#define CTLCU_CELL_MAXREG 48  // cell and pair sample loops: 5 blocks of 256 threads per SM
+#endif
+#ifndef CTLCU_SEGMENT_MAXREG
+#define CTLCU_SEGMENT_MAXREG 64  // segment loop: 4 blocks of 256 threads per SM
 #endif
 #ifndef CTLCU_GATHER_MAXREG
 #define CTLCU_GATHER_MAXREG 80  // gather, nearest-voxel and texture loops: 3 blocks of 256 per SM
@@ -36,7 +39,9 @@ constexpr int kPad = 2;
 // tile through nearly the same part of the volume, so their rays share cached
 // cells.  Each warp is a lanes_x x (32 / lanes_x) pixel patch of one view, so
 // its 32 rays are neighbours.  `unroll` samples of the cell and pair loops
-// form one FP32 partial sum before it goes to the accumulator.
+// form one FP32 partial sum before it goes to the accumulator; the segment loop,
+// whose segments hold about two samples each at the default step, takes unroll / 2
+// segments.
 struct LaunchShape {
     uint32_t block = 256;   // rays (threads) per block: 128, 256 or 512
     uint32_t views = 2;     // views per block: 1, 2 or 4
@@ -94,17 +99,31 @@ constexpr uint32_t kMagicBits = 0x4B400000u;
 constexpr int kCellBytes = 32;
 
 // Layout of the cell array of a volume with n voxels per axis: cells span
-// padded voxels, (n + 2 kPad - 1) per axis, x fastest, row stride sy, slice
-// stride sz.  sz is padded so that 1 + sy + sz is a multiple of 1024; then
-// kMagicBits * (1 + sy + sz) = 0 mod 2^32, and the index of the cell whose
-// per-axis magic sums have bit patterns bx, by, bz is exactly
-// bx + by sy + bz sz in 32-bit arithmetic.
+// padded voxels, (n + 2 kPad - 1) per axis.  Slices are stored in pairs: the two
+// z-neighbours of a pair lie next to each other, then x (stride 2), y (stride
+// sy), and the pairs (stride sz), with sy and sz = 2 mod 4.  The place of a cell
+// in its 128-byte line is then z + 2 x + 2 y mod 4.  A warp's 32-byte loads are
+// served four lanes at a time, and lanes whose cells differ but have the same
+// place are served one after the other (measured; lanes with the same cell, or
+// with different places in any lines, go together).  Four neighbouring detector
+// rows see cells that differ in z and by a step along the ray in x or y, which
+// this order puts into different places: 9.2 passes of the L1 data path per warp
+// load where x-fastest order with unpadded strides takes 12 to 14.
 struct CellLayout {
     uint32_t cx, cy, cz;  // cells per axis
-    uint32_t sy, sz;      // strides (cells) of y and of the slowest axis
+    uint32_t sy, sz;      // strides (cells) of y and of a pair of slices
     uint64_t count;       // cells allocated
-    uint32_t max_index;   // index of the last real cell
+    uint32_t max_index;   // last allocated cell
+    uint32_t offset;      // what cell_linear of magic-sum bit patterns has to add
 };
+
+// Linear cell index from per-axis indices, or from the bit patterns of their
+// magic sums with the layout's offset (32-bit arithmetic, which wraps).
+__host__ __device__ __forceinline__ uint32_t cell_linear(uint32_t ix, uint32_t iy, uint32_t iz, uint32_t sy,
+                                                         uint32_t sz, uint32_t offset)
+{
+    return (iz >> 1) * (sz - 2u) + offset + iy * sy + ix * 2u + iz;
+}
 
 inline CellLayout cell_layout(const int n[3])
 {
@@ -112,28 +131,23 @@ inline CellLayout cell_layout(const int n[3])
     L.cx = (uint32_t)(n[0] + 2 * kPad - 1);
     L.cy = (uint32_t)(n[1] + 2 * kPad - 1);
     L.cz = (uint32_t)(n[2] + 2 * kPad - 1);
-    L.sy = L.cx;
-    const uint32_t base = L.cx * L.cy;
-    const uint32_t e = (1024u - ((1u + L.sy + base) & 1023u)) & 1023u;
-    L.sz = base + e;
-    L.count = (uint64_t)L.sz * L.cz;
-    L.max_index = (L.cz - 1) * L.sz + (L.cy - 1) * L.sy + (L.cx - 1);
+    L.sy = 2 * L.cx + ((2u - 2 * L.cx) & 3u);
+    const uint32_t base = L.sy * L.cy;
+    L.sz = base + ((2u - base) & 3u);
+    L.count = (uint64_t)L.sz * ((L.cz + 1) / 2);
+    L.max_index = (uint32_t)(L.count - 1);
+    L.offset = 0u - cell_linear(kMagicBits, kMagicBits, kMagicBits, L.sy, L.sz, 0u);
     return L;
-}
-
-// Linear cell index from per-axis indices (or their magic-sum bit patterns).
-__host__ __device__ __forceinline__ uint32_t cell_linear(uint32_t ix, uint32_t iy, uint32_t iz, uint32_t sy,
-                                                         uint32_t sz)
-{
-    return ix + iy * sy + iz * sz;
 }
 
 // x-pair array: for every padded voxel (x < ext_x - 1, y, z) the float2
 // (mid, diff) = ((v[x] + v[x+1]) / 2, v[x+1] - v[x]), computed in FP64.  A
 // trilinear cell reads four entries (its two rows in y times two slices in
 // z); the x interpolation of an entry at offset h from the cell centre is
-// mid + h * diff.  8 bytes per voxel; strides padded like the cell array so
-// the magic offsets cancel.
+// mid + h * diff.  8 bytes per voxel; the slice stride is padded so that
+// 1 + sy + sz is a multiple of 1024: then kMagicBits * (1 + sy + sz) = 0 mod 2^32,
+// and the index of the entry whose per-axis magic sums have bit patterns bx, by,
+// bz is exactly bx + by sy + bz sz in 32-bit arithmetic.
 struct PairLayout {
     uint32_t px, ey, ez;  // entries per row, rows, slices
     uint32_t sy, sz;      // strides (entries)
@@ -156,7 +170,7 @@ inline PairLayout pair_layout(const int n[3])
     return L;
 }
 
-enum class Mode : int { Trilinear = 0, Nearest = 1, Texture = 2, Cells = 3, Pairs = 4 };
+enum class Mode : int { Trilinear = 0, Nearest = 1, Texture = 2, Cells = 3, Pairs = 4, Segments = 5 };
 enum class Accum : int { F64 = 0, Kahan = 1, F32 = 2 };
 
 // Everything a projection launch needs, passed by value.
@@ -170,15 +184,16 @@ struct ProjectArgs {
     double voxel[3];          // voxel size of that grid (mm)
     double corner[3];         // low corner of that grid (mm)
     double increment;         // step length (mm)
-    const void* cells;        // Mode::Cells: coefficient cells, x fastest
-    uint32_t csy, csz;        // cell strides (cells per row, per slice)
-    uint32_t cmax;            // last valid cell index
+    const void* cells;        // Mode::Cells and Segments: coefficient cells; Mode::Pairs: pair entries
+    uint32_t csy, csz;        // their strides (CellLayout, PairLayout)
+    uint32_t cmax;            // last valid index
+    uint32_t coffset;         // CellLayout::offset
     uint32_t vm_group;        // view groups per chunk of the block order
     uint32_t n_views;         // views (n_vm / n_modules)
     uint32_t view_groups;     // ceil(n_views / views per block)
     // launch shape (LaunchShape), as block size and log2 factors of the pixel mapping
     uint32_t block;           // threads per block
-    uint32_t unroll;          // samples per partial sum (cell and pair loops)
+    uint32_t unroll;          // samples per partial sum (cell and pair loops; segment loop: unroll / 2 segments)
     uint32_t vpb_shift;       // log2 views per block
     uint32_t wpv_shift;       // log2 warps per view
     uint32_t lx_shift;        // log2 lanes along the channels
@@ -211,10 +226,19 @@ struct BatchReq {
     uint32_t items;       // work items of this request
 };
 
+// Up to this ray_sampling the cells are read segment by segment, above it sample
+// by sample.  A segment costs about twice a sample, so it pays while it holds two
+// samples or so.  Segments / samples, ms, at ray_sampling 0.3, 0.5, 0.6, 0.75, 1:
+//   201x173x155 -> 23 x 479x361      2.00 / 2.99, 1.89 / 2.16, 1.83 / 1.92, 1.75 / 1.65, 1.55 / 1.33
+//   512^3 helical, 180 x 64 x 16^2   2.16 / 3.58, 2.05 / 2.75, 1.99 / 2.53, 1.90 / 2.25, 1.73 / 1.97
+// The rule looks at the setting alone, so that a request takes the same loop in a
+// batch as on its own.
+constexpr float kSegmentMaxSampling = 0.6f;
+
 // Launchers (raycast.cu / setup.cu / volume.cu).  All asynchronous on `s`.
 cudaError_t launch_batch_setup(const BatchSetup* reqs, uint32_t n_reqs, uint32_t total, ViewGeom* geom,
                                int* flags, cudaStream_t s);
-// Persistent launch (Mode::Cells or Mode::Pairs) over all work items of a
+// Persistent launch (Mode::Cells, Segments or Pairs) over all work items of a
 // batch (total_items block tiles, each block / 32 warp patches, dealt out to
 // warps one patch at a time), every request with the launch shape `shape`
 // (block size and unroll); `counter` must be zero at launch.  Returns the

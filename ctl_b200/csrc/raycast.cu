@@ -79,7 +79,7 @@ struct Accumulator<Accum::F32> {
     __device__ __forceinline__ double value() const { return static_cast<double>(s); }
 };
 
-// One ray ready for the sample loop.  The cell, pair and trilinear loops run in
+// One ray ready for the sample loop.  The cell, segment, pair and trilinear loops run in
 // FP32 relative to the ray's integer origin (CellFrame); the texture loop runs
 // from the rounded absolute base, its 8-bit filter weights being far coarser;
 // the nearest-voxel loop keeps FP64, because a position error there moves a
@@ -88,6 +88,7 @@ struct Ray {
     double base[3];  // coordinate of the first sample in the loop's index space
     double step[3];  // one step in voxel units
     int n;           // number of samples (0: the ray misses)
+    int first;       // index of the first sample (cell and segment loops)
 };
 
 // Face test of raycasterprojector_interp.cl:136-148.
@@ -147,7 +148,7 @@ __device__ __forceinline__ Ray setup_ray(const ProjectArgs& a, const ViewGeom& g
         r.step[0] = r.step[1] = r.step[2] = 0.0;
         return r;
     }
-    if (M == Mode::Cells || M == Mode::Pairs) {
+    if (M == Mode::Cells || M == Mode::Segments || M == Mode::Pairs) {
         // Only samples inside the box contribute (the reference's first and last
         // samples, floor(tmin) and floor(tmax)+1, lie outside it and read zeros),
         // so the loop runs over ceil(t0) .. floor(t1).  Coordinates are
@@ -155,6 +156,7 @@ __device__ __forceinline__ Ray setup_ray(const ProjectArgs& a, const ViewGeom& g
         // cell centre v - rint(v).
         const double i0 = ceil(t0), i1 = floor(t1);
         r.n = i1 >= i0 ? static_cast<int>(i1 - i0) + 1 : 0;
+        r.first = static_cast<int>(fmin(i0, 1.0e9));
         r.base[0] = (s0 - k0) + i0 * d0 + (kPad - 1.0);
         r.base[1] = (s1 - k1) + i0 * d1 + (kPad - 1.0);
         r.base[2] = (s2 - k2) + i0 * d2 + (kPad - 1.0);
@@ -339,7 +341,7 @@ __device__ __forceinline__ float cell_eval(const char* __restrict__ cells, uint3
 // already keep every sample inside it.
 __device__ __forceinline__ float2 cell_sample_pair(const char* __restrict__ cells, float2 kk, const CellFrame& fr,
                                                    float2 dx2, float2 dy2, float2 dz2, uint32_t sy, uint32_t sz,
-                                                   uint32_t cmax, CellCache& cc)
+                                                   uint32_t cmax, uint32_t offset, CellCache& cc)
 {
     const float2 none2 = make_float2(-1.0f, -1.0f);
     const float2 mx2 = make_float2(fr.mxy.x, fr.mxy.x), my2 = make_float2(fr.mxy.y, fr.mxy.y);
@@ -351,10 +353,10 @@ __device__ __forceinline__ float2 cell_sample_pair(const char* __restrict__ cell
     const float2 hx = __ffma2_rn(__ffma2_rn(mx2, none2, tx), none2, vx);  // v - (t - m)
     const float2 hy = __ffma2_rn(__ffma2_rn(my2, none2, ty), none2, vy);
     const float2 hz = __ffma2_rn(__ffma2_rn(mz2, none2, tz), none2, vz);
-    const uint32_t i0 = min(cell_linear(__float_as_uint(tx.x), __float_as_uint(ty.x), __float_as_uint(tz.x), sy, sz),
-                            cmax);
-    const uint32_t i1 = min(cell_linear(__float_as_uint(tx.y), __float_as_uint(ty.y), __float_as_uint(tz.y), sy, sz),
-                            cmax);
+    const uint32_t i0 = min(cell_linear(__float_as_uint(tx.x), __float_as_uint(ty.x), __float_as_uint(tz.x), sy, sz,
+                                        offset), cmax);
+    const uint32_t i1 = min(cell_linear(__float_as_uint(tx.y), __float_as_uint(ty.y), __float_as_uint(tz.y), sy, sz,
+                                        offset), cmax);
     const float f0 = cell_eval(cells, i0, hx.x, hy.x, hz.x, cc);
     const float f1 = cell_eval(cells, i1, hx.y, hy.y, hz.y, cc);
     return make_float2(f0, f1);
@@ -370,7 +372,7 @@ __device__ __forceinline__ void march_cells(const ProjectArgs& a, const Ray& r, 
     const float2 dx2 = make_float2((float)r.step[0], (float)r.step[0]);
     const float2 dy2 = make_float2((float)r.step[1], (float)r.step[1]);
     const float2 dz2 = make_float2((float)r.step[2], (float)r.step[2]);
-    const uint32_t sy = a.csy, sz = a.csz, cmax = a.cmax;
+    const uint32_t sy = a.csy, sz = a.csz, cmax = a.cmax, offset = a.coffset;
     const float2 two2 = make_float2(2.0f, 2.0f);
     float2 kk = make_float2(0.0f, 1.0f);  // steps k and k + 1
     CellCache cc;
@@ -379,7 +381,7 @@ __device__ __forceinline__ void march_cells(const ProjectArgs& a, const Ray& r, 
         float part = 0.0f;
 #pragma unroll
         for (int j = 0; j < U; j += 2) {
-            const float2 f = cell_sample_pair(cells, kk, fr, dx2, dy2, dz2, sy, sz, cmax, cc);
+            const float2 f = cell_sample_pair(cells, kk, fr, dx2, dy2, dz2, sy, sz, cmax, offset, cc);
             part += f.x;
             part += f.y;
             kk = __fadd2_rn(kk, two2);
@@ -391,13 +393,131 @@ __device__ __forceinline__ void march_cells(const ProjectArgs& a, const Ray& r, 
         // first value of a pair whose second step lies beyond the ray (its cell
         // index is clamped like any other, its value unused)
         for (; k + 1 < r.n; k += 2) {
-            const float2 f = cell_sample_pair(cells, kk, fr, dx2, dy2, dz2, sy, sz, cmax, cc);
+            const float2 f = cell_sample_pair(cells, kk, fr, dx2, dy2, dz2, sy, sz, cmax, offset, cc);
             acc.add(f.x);
             acc.add(f.y);
             kk = __fadd2_rn(kk, two2);
         }
         if (k < r.n)
-            acc.add(cell_sample_pair(cells, kk, fr, dx2, dy2, dz2, sy, sz, cmax, cc).x);
+            acc.add(cell_sample_pair(cells, kk, fr, dx2, dy2, dz2, sy, sz, cmax, offset, cc).x);
+    }
+}
+
+// Per-ray constants of the segment loop, one per axis: where the ray leaves a
+// cell (a sample at offset h from the cell's centre exits after e + h * i steps,
+// i = -1 / step, e = |i| / 2), and the products of two steps that weigh the
+// interpolant's mixed second derivatives, over 12.
+struct SegmentRay {
+    float2 ixy, exy;
+    float iz, ez;
+    float pxy, pxz, pyz;
+};
+
+__device__ __forceinline__ float exit_slope(float d)
+{
+    // an axis the ray does not move along (or by less than 1e-5 voxel over the
+    // longest ray) never ends a segment: its exit lies 5e11 steps away
+    return -1.0f / (fabsf(d) > 1.0e-12f ? d : copysignf(1.0e-12f, d));
+}
+
+__device__ __forceinline__ float min3(float a, float b, float c)
+{
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// One segment: the samples k, k + 1, .. last of a ray that lie in the cell of
+// sample k, summed in closed form.  On a line the interpolant of a cell is a
+// cubic in the step, and over samples placed evenly about their midpoint the odd
+// powers cancel, so m samples sum to
+//   m (f(mid) + (m^2 - 1) / 12 * q),
+//   q = dx dy f_xy(mid) + dx dz f_xz(mid) + dy dz f_yz(mid),
+// q being the quadratic coefficient (a trilinear interpolant has no f_xx).  The
+// position of sample k is formed as in cell_sample_pair; m follows from the exit
+// through the nearest face.  A sample within a rounding error of a face may be
+// counted to either side, where both interpolants agree to that error.  A lane
+// past its last sample (k = last + 1) gets m = 0 and adds nothing: its load stays
+// in the array and its values are not used.
+__device__ __forceinline__ void cell_segment(const char* __restrict__ cells, float& k, float last,
+                                             const CellFrame& fr, float2 dxy, float dz, const SegmentRay& sr,
+                                             uint32_t sy, uint32_t sz, uint32_t cmax, uint32_t offset, float& part)
+{
+    const float2 none2 = make_float2(-1.0f, -1.0f);
+    const float2 vxy = __ffma2_rn(make_float2(k, k), dxy, fr.bxy);
+    const float vz = fmaf(k, dz, fr.bz);
+    const float2 txy = __fadd2_rn(vxy, fr.mxy);
+    const float tz = __fadd_rn(vz, fr.mz);
+    const uint32_t idx = min(cell_linear(__float_as_uint(txy.x), __float_as_uint(txy.y), __float_as_uint(tz), sy, sz,
+                                         offset), cmax);
+    float c0, c1, c2, c3, c4, c5, c6, c7;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(c0), "=f"(c1), "=f"(c2), "=f"(c3), "=f"(c4), "=f"(c5), "=f"(c6), "=f"(c7)
+        : "l"(cells + (size_t)idx * kCellBytes));
+    const float2 hxy = __ffma2_rn(__ffma2_rn(fr.mxy, none2, txy), none2, vxy);  // v - (t - m)
+    const float hz = __fsub_rn(vz, __fsub_rn(tz, fr.mz));
+    // whole steps to the exit, none below 0 and at most to the last sample (-1 past it)
+    const float2 exy = __ffma2_rn(hxy, sr.ixy, sr.exy);
+    const float e = fminf(fmaxf(min3(exy.x, exy.y, fmaf(hz, sr.iz, sr.ez)), 0.0f), last - k);
+    const float m = __fadd_rd(e, 8388608.0f) - 8388607.0f;  // floor(e) + 1, e < kWindow
+    const float half = fmaf(m, 0.5f, -0.5f);
+    const float2 gxy = __ffma2_rn(make_float2(half, half), dxy, hxy);  // offsets of the midpoint
+    const float gz = fmaf(half, dz, hz);
+    const float2 hx2 = make_float2(gxy.x, gxy.x);
+    const float2 ea = __ffma2_rn(hx2, make_float2(c2, c3), make_float2(c0, c1));
+    const float2 eb = __ffma2_rn(hx2, make_float2(c6, c7), make_float2(c4, c5));
+    const float2 g = __ffma2_rn(make_float2(gxy.y, gxy.y), eb, ea);
+    const float f = fmaf(gz, g.y, g.x);
+    const float q = fmaf(sr.pyz, eb.y, fmaf(sr.pxz, fmaf(gxy.y, c7, c3), sr.pxy * fmaf(gz, c7, c6)));
+    if (k <= last)
+        part = fmaf(m, fmaf(fmaf(m, m, -1.0f), q, f), part);
+    k += m;
+}
+
+// Samples per window of the segment loop: the lanes of a warp, which step from
+// cell to cell each at its own pace, meet again at every sample index that is a
+// multiple of this.  Without that they drift apart by several cells along a long
+// ray, share fewer cells per load and conflict more in L1 (256^3 -> 60 x 512^2
+// with windows of 32, 64, 128, 256 samples and none: 12.6, 11.6, 11.3, 11.2 and
+// 11.7 ms; 512^3 helical: 2.31, 2.20, 2.17, 2.18 and 2.36 ms).
+constexpr int kWindow = 128;
+
+// Sample sum by segments: one cell load and one evaluation per cell in which a
+// ray has samples, instead of per sample; U segments per FP32 partial sum.  At
+// the default step (0.3 voxel) a segment holds 2.4 samples on average.  Called by
+// all 32 lanes of a warp (r.n = 0 for a lane without a ray).  The windows lie at
+// fixed sample indexes, so a ray's segments and partial sums do not depend on the
+// warp that runs it.
+template <Accum ACC, int U>
+__device__ __forceinline__ void march_segments(const ProjectArgs& a, const Ray& r, Accumulator<ACC>& acc)
+{
+    const char* __restrict__ cells = static_cast<const char*>(a.cells);
+    const CellFrame fr = cell_frame(r);
+    const float2 dxy = make_float2((float)r.step[0], (float)r.step[1]);
+    const float dz = (float)r.step[2];
+    SegmentRay sr;
+    sr.ixy = make_float2(exit_slope(dxy.x), exit_slope(dxy.y));
+    sr.iz = exit_slope(dz);
+    sr.exy = make_float2(0.5f * fabsf(sr.ixy.x), 0.5f * fabsf(sr.ixy.y));
+    sr.ez = 0.5f * fabsf(sr.iz);
+    sr.pxy = dxy.x * dxy.y * (1.0f / 12.0f);
+    sr.pxz = dxy.x * dz * (1.0f / 12.0f);
+    sr.pyz = dxy.y * dz * (1.0f / 12.0f);
+    const uint32_t sy = a.csy, sz = a.csz, cmax = a.cmax, offset = a.coffset;
+    const bool hit = r.n > 0;
+    const int w1 = __reduce_max_sync(0xffffffffu, hit ? (r.first + r.n - 1) / kWindow : -1);
+    int w = __reduce_min_sync(0xffffffffu, hit ? r.first / kWindow : 0x7fffffff);
+    float k = 0.0f;
+    for (; w <= w1; ++w) {
+        const float last = (float)(min(r.n, (w + 1) * kWindow - r.first) - 1);
+        while (k <= last) {
+            float part = 0.0f;
+#pragma unroll
+            for (int j = 0; j < U; ++j)
+                cell_segment(cells, k, last, fr, dxy, dz, sr, sy, sz, cmax, offset, part);
+            acc.add(part);
+        }
+        __syncwarp();
     }
 }
 
@@ -513,9 +633,11 @@ __device__ __forceinline__ bool pixel_of_item(const ProjectArgs& a, uint32_t b, 
     const uint32_t view = (vg << a.vpb_shift) + slot;
     vm = view * a.n_modules + m;
     const uint32_t ty = t / a.tiles_x, tx = t - ty * a.tiles_x;
+    // consecutive lanes run down the rows of a channel: their rays share x and y and
+    // differ in z, which the cell layout serves without conflicts (CellLayout)
     const uint32_t ly_shift = 5u - a.lx_shift;
-    x = (tx << a.tx_shift) + ((w & ((1u << a.wx_shift) - 1u)) << a.lx_shift) + (lane & ((1u << a.lx_shift) - 1u));
-    y = (ty << a.ty_shift) + ((w >> a.wx_shift) << ly_shift) + (lane >> a.lx_shift);
+    x = (tx << a.tx_shift) + ((w & ((1u << a.wx_shift) - 1u)) << a.lx_shift) + (lane >> ly_shift);
+    y = (ty << a.ty_shift) + ((w >> a.wx_shift) << ly_shift) + (lane & ((1u << ly_shift) - 1u));
     return view < a.n_views && x < a.channels && y < a.rows;
 }
 
@@ -531,23 +653,26 @@ __device__ __forceinline__ bool pixel_of(const ProjectArgs& a, uint32_t& vm, uin
 }
 
 // Writes the warp's pixel values (called by all 32 lanes): each lane holds
-// `val` for pixel (vm, x, y), or ok = false for no pixel.  Four consecutive
-// lanes are four consecutive channels of one detector row (a warp patch is 4
-// or 8 channels wide), so where all four pixels exist and their row segment
-// starts on a 16-byte boundary, the quad's first lane gathers the other three
-// values and writes the segment as one 16-byte store; otherwise each lane
-// stores its own value.
+// `val` for pixel (vm, x, y), or ok = false for no pixel.  The lanes of four
+// consecutive channels of one detector row lie one patch height apart (a warp
+// patch is 4 or 8 channels wide); where all four pixels exist and their row
+// segment starts on a 16-byte boundary, the first of them gathers the other three
+// values and writes the segment as one 16-byte store; otherwise each lane stores
+// its own value.
 __device__ __forceinline__ void store_patch(const ProjectArgs& a, uint32_t vm, uint32_t x, uint32_t y, float val,
                                             bool ok)
 {
-    const uint32_t full = 0xffffffffu, lane = threadIdx.x & 31u, lead = lane & ~3u;
-    const float v1 = __shfl_down_sync(full, val, 1);
-    const float v2 = __shfl_down_sync(full, val, 2);
-    const float v3 = __shfl_down_sync(full, val, 3);
+    const uint32_t full = 0xffffffffu, lane = threadIdx.x & 31u;
+    const uint32_t ls = 5u - a.lx_shift;  // log2 of the patch height
+    const uint32_t lead = lane & ~(3u << ls);
+    const float v1 = __shfl_down_sync(full, val, 1u << ls);
+    const float v2 = __shfl_down_sync(full, val, 2u << ls);
+    const float v3 = __shfl_down_sync(full, val, 3u << ls);
     const uint32_t okmask = __ballot_sync(full, ok);
+    const uint32_t quad = 1u | (1u << (1u << ls)) | (1u << (2u << ls)) | (1u << (3u << ls));
     float* dst = a.out + ((size_t)vm * a.rows + y) * a.channels + x;
-    const bool whole = ((okmask >> lead) & 0xfu) == 0xfu && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0;
-    // the quad's choice is its first lane's
+    const bool whole = ((okmask >> lead) & quad) == quad && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0;
+    // the choice of the four is their first lane's
     const bool vec = __shfl_sync(full, whole ? 1 : 0, lead) != 0;
     if (vec) {
         if (lane == lead)
@@ -557,51 +682,61 @@ __device__ __forceinline__ void store_patch(const ProjectArgs& a, uint32_t vm, u
     }
 }
 
-// The rays of work item `b` for thread `tid`, cell or pair loop (FP32 entries).
-// Called by every lane of a warp (the store is warp-cooperative).
+// The sample loop of a derived array's mode.
+template <Mode M, Accum ACC, int U>
+__device__ __forceinline__ void march_array(const ProjectArgs& a, const Ray& r, Accumulator<ACC>& acc)
+{
+    if (M == Mode::Pairs)
+        march_pairs<ACC, U>(a, r, acc);
+    else if (M == Mode::Segments)
+        march_segments<ACC, U>(a, r, acc);
+    else
+        march_cells<ACC, U>(a, r, acc);
+}
+
+// The rays of work item `b` for thread `tid`, cell, segment or pair loop (FP32
+// entries).  Called by every lane of a warp (the segment loop and the store are
+// warp-cooperative): a lane without a pixel or with an unusable matrix marches a
+// ray of no samples.
 template <Mode M, Accum ACC, int U>
 __device__ __forceinline__ void cells_item(const ProjectArgs& a, uint32_t b, uint32_t tid)
 {
     uint32_t vm, x, y;
     const bool ok = pixel_of_item(a, b, tid, vm, x, y);
-    float val = 0.0f;
-    if (ok) {
-        const ViewGeom& g = a.geom[vm];
-        if (g.valid) {
-            Accumulator<ACC> acc;
-            if (a.rays_x == 1 && a.rays_y == 1) {
-                // one ray through the pixel centre (x - 0.5 + 0.5 is x exactly): the
-                // pixel and its geometry are dead once the ray is set up, so the
-                // sample loop carries only the ray
-                const Ray r = setup_ray<M>(a, g, (double)x, (double)y, a.flags);
-                if (M == Mode::Pairs)
-                    march_pairs<ACC, U>(a, r, acc);
-                else
-                    march_cells<ACC, U>(a, r, acc);
-            } else {
-                const double ix = 1.0 / a.rays_x, iy = 1.0 / a.rays_y;
-                for (uint32_t rx = 0; rx < a.rays_x; ++rx)
-                    for (uint32_t ry = 0; ry < a.rays_y; ++ry) {
-                        const double px = (double)x - 0.5 + 0.5 * ix + rx * ix;
-                        const double py = (double)y - 0.5 + 0.5 * iy + ry * iy;
-                        const Ray r = setup_ray<M>(a, g, px, py, a.flags);
-                        if (M == Mode::Pairs)
-                            march_pairs<ACC, U>(a, r, acc);
-                        else
-                            march_cells<ACC, U>(a, r, acc);
-                    }
+    const ViewGeom& g = a.geom[ok ? vm : 0u];
+    const bool live = ok && g.valid;
+    Accumulator<ACC> acc;
+    if (a.rays_x == 1 && a.rays_y == 1) {
+        // one ray through the pixel centre (x - 0.5 + 0.5 is x exactly): the
+        // pixel and its geometry are dead once the ray is set up, so the
+        // sample loop carries only the ray
+        Ray r = setup_ray<M>(a, g, (double)x, (double)y, live ? a.flags : nullptr);
+        if (!live)
+            r.n = 0;
+        march_array<M, ACC, U>(a, r, acc);
+    } else {
+        const double ix = 1.0 / a.rays_x, iy = 1.0 / a.rays_y;
+        for (uint32_t rx = 0; rx < a.rays_x; ++rx)
+            for (uint32_t ry = 0; ry < a.rays_y; ++ry) {
+                const double px = (double)x - 0.5 + 0.5 * ix + rx * ix;
+                const double py = (double)y - 0.5 + 0.5 * iy + ry * iy;
+                Ray r = setup_ray<M>(a, g, px, py, live ? a.flags : nullptr);
+                if (!live)
+                    r.n = 0;
+                march_array<M, ACC, U>(a, r, acc);
             }
-            val = static_cast<float>(a.increment * acc.value() / (double)(a.rays_x * a.rays_y));
-        }
     }
+    const float val = static_cast<float>(a.increment * acc.value() / (double)(a.rays_x * a.rays_y));
     // the pixel again for the store, rather than holding it through the loop
     pixel_of_item(a, b, tid, vm, x, y);
     store_patch(a, vm, x, y, val, ok);
 }
 
-// Cell or pair loop over one block of the regular grid.
+constexpr int cell_maxreg(Mode m) { return m == Mode::Segments ? CTLCU_SEGMENT_MAXREG : CTLCU_CELL_MAXREG; }
+
+// Cell, segment or pair loop over one block of the regular grid.
 template <Mode M, Accum ACC, int U>
-__global__ void __maxnreg__(CTLCU_CELL_MAXREG) cells_kernel(const ProjectArgs a)
+__global__ void __maxnreg__(cell_maxreg(M)) cells_kernel(const ProjectArgs a)
 {
     cells_item<M, ACC, U>(a, blockIdx.x, threadIdx.x);
 }
@@ -621,7 +756,7 @@ __global__ void __maxnreg__(CTLCU_CELL_MAXREG) cells_kernel(const ProjectArgs a)
 // changes.
 
 template <Mode M, Accum ACC, int U>
-__global__ void __maxnreg__(CTLCU_CELL_MAXREG)
+__global__ void __maxnreg__(cell_maxreg(M))
     batch_cells_kernel(const BatchReq* __restrict__ reqs, uint32_t n_reqs, uint32_t total_warp_items,
                        uint32_t wpb_shift, unsigned int* counter)
 {
@@ -728,13 +863,16 @@ cudaError_t launch_typed(const ProjectArgs& a, int dtype, dim3 grid, cudaStream_
     return cudaGetLastError();
 }
 
+// Samples, or segments of about two samples, per partial sum of a loop.
+constexpr int loop_unroll(Mode m, int unroll) { return m == Mode::Segments ? unroll / 2 : unroll; }
+
 template <Mode M, Accum ACC>
 cudaError_t launch_cells(const ProjectArgs& a, dim3 grid, cudaStream_t s)
 {
     switch (a.unroll) {
-    case 2: cells_kernel<M, ACC, 2><<<grid, a.block, 0, s>>>(a); break;
-    case 4: cells_kernel<M, ACC, 4><<<grid, a.block, 0, s>>>(a); break;
-    case 8: cells_kernel<M, ACC, 8><<<grid, a.block, 0, s>>>(a); break;
+    case 2: cells_kernel<M, ACC, loop_unroll(M, 2)><<<grid, a.block, 0, s>>>(a); break;
+    case 4: cells_kernel<M, ACC, loop_unroll(M, 4)><<<grid, a.block, 0, s>>>(a); break;
+    case 8: cells_kernel<M, ACC, loop_unroll(M, 8)><<<grid, a.block, 0, s>>>(a); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -752,6 +890,7 @@ cudaError_t launch_acc(const ProjectArgs& a, Mode mode, int dtype, dim3 grid, cu
         project_kernel<float, Mode::Texture, ACC, false><<<grid, a.block, 0, s>>>(a);
         return cudaGetLastError();
     case Mode::Cells: return launch_cells<Mode::Cells, ACC>(a, grid, s);
+    case Mode::Segments: return launch_cells<Mode::Segments, ACC>(a, grid, s);
     case Mode::Pairs: return launch_cells<Mode::Pairs, ACC>(a, grid, s);
     }
     return cudaErrorInvalidValue;
@@ -809,9 +948,9 @@ cudaError_t launch_batch_unroll(const BatchReq* reqs, uint32_t n_reqs, uint32_t 
                                 unsigned int* counter, int* blocks, cudaStream_t s)
 {
     switch (sh.unroll) {
-    case 2: return launch_batch_typed<M, ACC, 2>(reqs, n_reqs, total, sh.block, counter, blocks, s);
-    case 4: return launch_batch_typed<M, ACC, 4>(reqs, n_reqs, total, sh.block, counter, blocks, s);
-    case 8: return launch_batch_typed<M, ACC, 8>(reqs, n_reqs, total, sh.block, counter, blocks, s);
+    case 2: return launch_batch_typed<M, ACC, loop_unroll(M, 2)>(reqs, n_reqs, total, sh.block, counter, blocks, s);
+    case 4: return launch_batch_typed<M, ACC, loop_unroll(M, 4)>(reqs, n_reqs, total, sh.block, counter, blocks, s);
+    case 8: return launch_batch_typed<M, ACC, loop_unroll(M, 8)>(reqs, n_reqs, total, sh.block, counter, blocks, s);
     }
     return cudaErrorInvalidValue;
 }
@@ -840,6 +979,8 @@ cudaError_t launch_batch(const BatchReq* reqs, uint32_t n_reqs, uint32_t total_i
         return launch_batch_mode<Mode::Pairs>(reqs, n_reqs, total_items, acc, shape, counter, blocks, s);
     if (mode == Mode::Cells)
         return launch_batch_mode<Mode::Cells>(reqs, n_reqs, total_items, acc, shape, counter, blocks, s);
+    if (mode == Mode::Segments)
+        return launch_batch_mode<Mode::Segments>(reqs, n_reqs, total_items, acc, shape, counter, blocks, s);
     return cudaErrorInvalidValue;
 }
 

@@ -67,10 +67,12 @@ typedef enum {
  * Sample-loop variant.  AUTO picks CELLS for software trilinear interpolation
  * without up-sampling and GATHER otherwise.
  *   GATHER  eight scalar loads per sample from the zero-padded voxel array
- *   CELLS   one 32-byte load per sample from a derived cell array holding,
- *           per trilinear cell, the 8 coefficients of its interpolation
- *           polynomial about the cell centre (FP32, built on the device once
- *           per resident volume; 8x the voxel count x 4 bytes)
+ *   CELLS   32-byte loads from a derived cell array holding, per trilinear cell,
+ *           the 8 coefficients of its interpolation polynomial about the cell
+ *           centre (FP32, built on the device once per resident volume; 8x the
+ *           voxel count x 4 bytes).  Up to ray_sampling 0.6 the samples a ray
+ *           has in a cell are summed in closed form (one load and one evaluation
+ *           per cell); above it, sample by sample
  */
 typedef enum {
     CTLCU_KERNEL_AUTO = 0,
@@ -114,7 +116,8 @@ typedef struct {
     int32_t block_rays;         /* rays (threads) per block: 128, 256 or 512 [256]; the tile is
                                    block_rays/views_per_block pixels, 16 channels wide from 128
                                    pixels up, else 8 */
-    int32_t unroll;             /* cell/pair loops: samples per FP32 partial sum, 2, 4 or 8 [4] */
+    int32_t unroll;             /* cell/pair loops: samples per FP32 partial sum, 2, 4 or 8 [4]; summed by
+                                   cells: unroll/2 cells of about two samples each */
 } ctlcu_settings;
 
 /* One projection request of a batch: device pointers, see ctlcu_project_batch. */

@@ -1,0 +1,78 @@
+"""The cell loop that sums a ray's samples cell by cell, at the sizes where it can
+go wrong: volumes of one voxel to several hundred along the rays (no sample in the
+box, one window of samples, several), rays along an axis or nearly so, partial
+warps, and sampling steps on both sides of the line between this loop and the
+sample-by-sample one.  Bar: the parity bar of the projector (1e-4 of the value or
+of a thousandth of the maximum, tests/_common.py)."""
+import numpy as np
+import pytest
+
+import oracle
+from _common import rel_err
+from ctl_b200 import _lib as L
+from ctl_b200 import geometry as G
+from ctl_b200.projector import Context, Settings, VoxelVolume
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    with Context(0) as c:
+        yield c
+
+
+def _volume(shape_xyz, seed):
+    rng = np.random.default_rng(seed)
+    return (rng.uniform(0.01, 0.05, shape_xyz[::-1]) * (rng.random(shape_xyz[::-1]) < 0.8)).astype(np.float32)
+
+
+def _axis_views(channels, rows, pitch, tilt):
+    """Views from +x, +y and (nearly) +z, `tilt` rad off each axis."""
+    out = []
+    for axis in range(3):
+        d = np.full(3, tilt)
+        d[axis] = 1.0
+        up = np.array([0.0, 0.0, 1.0]) if axis < 2 else np.array([1.0, 0.0, 0.0])
+        R = G.camera_rotation(-d, up)
+        K = G.intrinsic(1200.0, pitch, pitch, (channels - 1) / 2, (rows - 1) / 2)
+        out.append(G.normalized(G.compose(K, R, 900.0 * d / np.linalg.norm(d))))
+    return np.stack(out)[:, None]
+
+
+@pytest.mark.parametrize("sampling", [0.05, 0.3, 0.6, 0.61, 1.0, 2.5])
+@pytest.mark.parametrize("shape,voxel", [((1, 1, 1), (30.0, 30.0, 30.0)), ((2, 3, 127), (20.0, 15.0, 1.0)),
+                                         ((43, 42, 5), (1.0, 1.0, 7.0)), ((300, 6, 5), (0.5, 6.0, 7.0))])
+@pytest.mark.parametrize("tilt", [0.0, 1e-7, 0.31])
+def test_cell_sums_match_the_oracle(ctx, shape, voxel, sampling, tilt):
+    vol = _volume(shape, 3)
+    C, R = 37, 21
+    P = _axis_views(C, R, 1.9, tilt)
+    want, _ = oracle.project_fp64(vol, voxel, P, C, R, ray_sampling=sampling)
+    v = ctx.volume(VoxelVolume(vol, voxel))
+    try:
+        for accum in (L.ACCUM_KAHAN, L.ACCUM_FP64):
+            got = ctx.project(v, P, C, R, Settings(ray_sampling=sampling, accum=accum, kernel=L.KERNEL_CELLS))
+            assert want.max() > 0
+            assert rel_err(got, want).max() <= 1e-4
+    finally:
+        v.release()
+
+
+def test_unusable_matrix_and_partial_warps_leave_the_other_pixels_alone(ctx):
+    """A singular view between good ones in one block: its pixels are 0, the others as without it."""
+    vol = _volume((20, 18, 16), 5)
+    P = _axis_views(11, 7, 4.0, 0.2)
+    bad = P.copy()
+    bad[1] = 0.0
+    v = ctx.volume(VoxelVolume(vol, (2.0, 2.0, 2.0)))
+    try:
+        good = ctx.project(v, P, 11, 7, Settings())
+        out = np.empty_like(good)
+        with pytest.raises(L.CtlcuError) as e:
+            ctx.project(v, bad, 11, 7, Settings(), out=out)
+        assert e.value.status == L.ERR_SINGULAR_GEOMETRY
+        np.testing.assert_array_equal(out[1], 0.0)
+        np.testing.assert_array_equal(out[[0, 2]], good[[0, 2]])
+    finally:
+        v.release()
