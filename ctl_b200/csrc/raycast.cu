@@ -69,7 +69,8 @@ struct Accumulator<Accum::Kahan> {
         c = (t - s) - y;
         s = t;
     }
-    __device__ __forceinline__ double value() const { return static_cast<double>(s); }
+    // the compensation still holds what the last additions rounded off s
+    __device__ __forceinline__ double value() const { return static_cast<double>(s) - static_cast<double>(c); }
 };
 
 template <>
@@ -474,27 +475,46 @@ __device__ __forceinline__ void cell_segment(const char* __restrict__ cells, flo
     k += m;
 }
 
+// One axis of a frame moved on by K steps: K d + (K dl) is formed with its FP32
+// rounding error, d + dl being the step to twice FP32's precision, and the integer
+// part of the new position goes into m, the remainder (about [-1/2, 1/2]) into b.
+__device__ __forceinline__ void advance_axis(float& b, float& m, float d, float dl, float K)
+{
+    const float p = __fmul_rn(K, d);
+    const float low = fmaf(K, dl, fmaf(K, d, -p));
+    const float t = __fadd_rn(p, m);
+    const float u = __fadd_rn(__fsub_rn(p, __fsub_rn(t, m)), __fadd_rn(b, low));
+    m = __fadd_rn(u, t);
+    b = __fsub_rn(u, __fsub_rn(m, t));
+}
+
 // Samples per window of the segment loop: the lanes of a warp, which step from
 // cell to cell each at its own pace, meet again at every sample index that is a
-// multiple of this.  Without that they drift apart by several cells along a long
+// multiple of this, where positions are also formed anew (advance_axis).  Without that they drift apart by several cells along a long
 // ray, share fewer cells per load and conflict more in L1 (256^3 -> 60 x 512^2
-// with windows of 32, 64, 128, 256 samples and none: 12.6, 11.6, 11.3, 11.2 and
-// 11.7 ms; 512^3 helical: 2.31, 2.20, 2.17, 2.18 and 2.36 ms).
-constexpr int kWindow = 128;
+// with windows of 128, 192 and 256 samples: 11.48, 11.26 and 11.39 ms; 512^3
+// helical, 180 views: 2.18, 2.17 and 2.19 ms.  Before positions were formed anew at
+// the windows: 32, 64, 128 samples and no windows 12.6, 11.6, 11.3 and 11.7 ms).
+constexpr int kWindow = 192;
 
 // Sample sum by segments: one cell load and one evaluation per cell in which a
 // ray has samples, instead of per sample; U segments per FP32 partial sum.  At
 // the default step (0.3 voxel) a segment holds 2.4 samples on average.  Called by
 // all 32 lanes of a warp (r.n = 0 for a lane without a ray).  The windows lie at
 // fixed sample indexes, so a ray's segments and partial sums do not depend on the
-// warp that runs it.
+// warp that runs it.  Steps count from the start of the window, whose position is
+// carried in more than FP32, so positions and step lengths stay exact to 1e-6 voxel
+// along the whole ray (2-norm error against 64 bits at 201x173x155: 2.8e-8, of
+// which 2.5e-8 is the rounding of the result; 5.2e-8 with steps counted from the
+// ray's start).
 template <Accum ACC, int U>
 __device__ __forceinline__ void march_segments(const ProjectArgs& a, const Ray& r, Accumulator<ACC>& acc)
 {
     const char* __restrict__ cells = static_cast<const char*>(a.cells);
-    const CellFrame fr = cell_frame(r);
+    CellFrame fr = cell_frame(r);
     const float2 dxy = make_float2((float)r.step[0], (float)r.step[1]);
     const float dz = (float)r.step[2];
+    const float lx = (float)(r.step[0] - dxy.x), ly = (float)(r.step[1] - dxy.y), lz = (float)(r.step[2] - dz);
     SegmentRay sr;
     sr.ixy = make_float2(exit_slope(dxy.x), exit_slope(dxy.y));
     sr.iz = exit_slope(dz);
@@ -507,15 +527,24 @@ __device__ __forceinline__ void march_segments(const ProjectArgs& a, const Ray& 
     const bool hit = r.n > 0;
     const int w1 = __reduce_max_sync(0xffffffffu, hit ? (r.first + r.n - 1) / kWindow : -1);
     int w = __reduce_min_sync(0xffffffffu, hit ? r.first / kWindow : 0x7fffffff);
-    float k = 0.0f;
+    int at = r.first;                   // the lane's next sample
+    const int end = r.first + r.n;
     for (; w <= w1; ++w) {
-        const float last = (float)(min(r.n, (w + 1) * kWindow - r.first) - 1);
-        while (k <= last) {
-            float part = 0.0f;
+        const int stop = min(end, (w + 1) * kWindow);
+        if (at < stop) {
+            const float last = (float)(stop - at - 1);
+            float k = 0.0f;
+            do {
+                float part = 0.0f;
 #pragma unroll
-            for (int j = 0; j < U; ++j)
-                cell_segment(cells, k, last, fr, dxy, dz, sr, sy, sz, cmax, offset, part);
-            acc.add(part);
+                for (int j = 0; j < U; ++j)
+                    cell_segment(cells, k, last, fr, dxy, dz, sr, sy, sz, cmax, offset, part);
+                acc.add(part);
+            } while (k <= last);
+            advance_axis(fr.bxy.x, fr.mxy.x, dxy.x, lx, k);
+            advance_axis(fr.bxy.y, fr.mxy.y, dxy.y, ly, k);
+            advance_axis(fr.bz, fr.mz, dz, lz, k);
+            at = stop;
         }
         __syncwarp();
     }
