@@ -726,7 +726,15 @@ int project_any(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, const d
             CU_TRY(ctx, cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
         if (!ctx->aux_stream)
             CU_TRY(ctx, cudaStreamCreateWithFlags(&ctx->aux_stream, cudaStreamNonBlocking));
-        // the second stream starts after the pmats upload and the volume staging on `st`
+        // the second stream starts after the pmats upload, the volume staging and
+        // the derived arrays, which are built here rather than by the first chunk
+        {
+            const ctlcu_settings eff = resolve_kernel(ctx, v, s, C, R, M);
+            ProjectArgs a = {};
+            Mode mode;
+            int dtype;
+            r = volume_args(ctx, v, &eff, a, mode, dtype);
+        }
         CU_TRY(ctx, cudaEventRecord(ctx->order, st));
         CU_TRY(ctx, cudaStreamWaitEvent(ctx->aux_stream, ctx->order, 0));
         const cudaStream_t lanes[2] = { st, ctx->aux_stream };
