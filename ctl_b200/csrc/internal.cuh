@@ -22,7 +22,7 @@ constexpr int kPad = 2;
 #define CTLCU_CELL_MAXREG 48  // cell and pair sample loops: 5 blocks of 256 threads per SM
 #endif
 #ifndef CTLCU_SEGMENT_MAXREG
-#define CTLCU_SEGMENT_MAXREG 64  // segment loop: 4 blocks of 256 threads per SM
+#define CTLCU_SEGMENT_MAXREG 64  // segment and up-sampled cell loops: 4 blocks of 256 threads per SM
 #endif
 #ifndef CTLCU_GATHER_MAXREG
 #define CTLCU_GATHER_MAXREG 80  // gather, nearest-voxel and texture loops: 3 blocks of 256 per SM
@@ -170,7 +170,7 @@ inline PairLayout pair_layout(const int n[3])
     return L;
 }
 
-enum class Mode : int { Trilinear = 0, Nearest = 1, Texture = 2, Cells = 3, Pairs = 4, Segments = 5 };
+enum class Mode : int { Trilinear = 0, Nearest = 1, Texture = 2, Cells = 3, Pairs = 4, Segments = 5, CellsUp = 6 };
 enum class Accum : int { F64 = 0, Kahan = 1, F32 = 2 };
 
 // Everything a projection launch needs, passed by value.
@@ -184,7 +184,7 @@ struct ProjectArgs {
     double voxel[3];          // voxel size of that grid (mm)
     double corner[3];         // low corner of that grid (mm)
     double increment;         // step length (mm)
-    const void* cells;        // Mode::Cells and Segments: coefficient cells; Mode::Pairs: pair entries
+    const void* cells;        // Mode::Cells, Segments and CellsUp: coefficient cells; Mode::Pairs: pair entries
     uint32_t csy, csz;        // their strides (CellLayout, PairLayout)
     uint32_t cmax;            // last valid index
     uint32_t coffset;         // CellLayout::offset

@@ -149,7 +149,7 @@ __device__ __forceinline__ Ray setup_ray(const ProjectArgs& a, const ViewGeom& g
         r.step[0] = r.step[1] = r.step[2] = 0.0;
         return r;
     }
-    if (M == Mode::Cells || M == Mode::Segments || M == Mode::Pairs) {
+    if (M == Mode::Cells || M == Mode::Segments || M == Mode::Pairs || M == Mode::CellsUp) {
         // Only samples inside the box contribute (the reference's first and last
         // samples, floor(tmin) and floor(tmax)+1, lie outside it and read zeros),
         // so the loop runs over ceil(t0) .. floor(t1).  Coordinates are
@@ -164,6 +164,16 @@ __device__ __forceinline__ Ray setup_ray(const ProjectArgs& a, const ViewGeom& g
         r.step[0] = d0;
         r.step[1] = d1;
         r.step[2] = d2;
+        if (M == Mode::CellsUp) {
+            // the same in stored voxels, a.up of the grid's to one
+            const double f = a.up;
+            r.base[0] = ((s0 - k0) + i0 * d0) / f + (kPad - 1.0);
+            r.base[1] = ((s1 - k1) + i0 * d1) / f + (kPad - 1.0);
+            r.base[2] = ((s2 - k2) + i0 * d2) / f + (kPad - 1.0);
+            r.step[0] = d0 / f;
+            r.step[1] = d1 / f;
+            r.step[2] = d2 / f;
+        }
         return r;
     }
     const double i0 = floor(t0), i1 = floor(t1) + 1.0;
@@ -332,6 +342,12 @@ __device__ __forceinline__ float cell_eval(const char* __restrict__ cells, uint3
     return fmaf(hz, g.y, g.x);
 }
 
+// up * h held to [-1/2, 1/2]
+__device__ __forceinline__ float2 hold_half(float2 h, float up)
+{
+    return make_float2(__saturatef(fmaf(up, h.x, 0.5f)) - 0.5f, __saturatef(fmaf(up, h.y, 0.5f)) - 0.5f);
+}
+
 // Two consecutive samples of a ray (steps k and k + 1, the lanes of kk) from
 // the coefficient cells.  Per axis: v' = (base - I) + k step; t = v' + m rounds
 // to the cell index (its bits minus kMagicBits, see CellFrame); h = v' - (t - m)
@@ -340,9 +356,15 @@ __device__ __forceinline__ float cell_eval(const char* __restrict__ cells, uint3
 // between two cells may take either of them; both give the same interpolated
 // value.  The cell index is clamped to the array as a guard; the loop bounds
 // already keep every sample inside it.
+//
+// UP (virtual f^3 replication, f = up): between the centres of two stored
+// voxels the replicated grid is flat but for one grid voxel about the face between
+// them, where it rises linearly.  Along each axis that is the cell's own
+// interpolant at f h instead of h, held at -1/2 and 1/2.
+template <bool UP>
 __device__ __forceinline__ float2 cell_sample_pair(const char* __restrict__ cells, float2 kk, const CellFrame& fr,
                                                    float2 dx2, float2 dy2, float2 dz2, uint32_t sy, uint32_t sz,
-                                                   uint32_t cmax, uint32_t offset, CellCache& cc)
+                                                   uint32_t cmax, uint32_t offset, float up, CellCache& cc)
 {
     const float2 none2 = make_float2(-1.0f, -1.0f);
     const float2 mx2 = make_float2(fr.mxy.x, fr.mxy.x), my2 = make_float2(fr.mxy.y, fr.mxy.y);
@@ -351,9 +373,14 @@ __device__ __forceinline__ float2 cell_sample_pair(const char* __restrict__ cell
     const float2 vy = __ffma2_rn(kk, dy2, make_float2(fr.bxy.y, fr.bxy.y));
     const float2 vz = __ffma2_rn(kk, dz2, make_float2(fr.bz, fr.bz));
     const float2 tx = __fadd2_rn(vx, mx2), ty = __fadd2_rn(vy, my2), tz = __fadd2_rn(vz, mz2);
-    const float2 hx = __ffma2_rn(__ffma2_rn(mx2, none2, tx), none2, vx);  // v - (t - m)
-    const float2 hy = __ffma2_rn(__ffma2_rn(my2, none2, ty), none2, vy);
-    const float2 hz = __ffma2_rn(__ffma2_rn(mz2, none2, tz), none2, vz);
+    float2 hx = __ffma2_rn(__ffma2_rn(mx2, none2, tx), none2, vx);  // v - (t - m)
+    float2 hy = __ffma2_rn(__ffma2_rn(my2, none2, ty), none2, vy);
+    float2 hz = __ffma2_rn(__ffma2_rn(mz2, none2, tz), none2, vz);
+    if (UP) {
+        hx = hold_half(hx, up);
+        hy = hold_half(hy, up);
+        hz = hold_half(hz, up);
+    }
     const uint32_t i0 = min(cell_linear(__float_as_uint(tx.x), __float_as_uint(ty.x), __float_as_uint(tz.x), sy, sz,
                                         offset), cmax);
     const uint32_t i1 = min(cell_linear(__float_as_uint(tx.y), __float_as_uint(ty.y), __float_as_uint(tz.y), sy, sz,
@@ -365,7 +392,7 @@ __device__ __forceinline__ float2 cell_sample_pair(const char* __restrict__ cell
 
 // Sample loop over the coefficient cells, U samples per partial sum (FP32)
 // handed to the accumulator.
-template <Accum ACC, int U>
+template <Accum ACC, int U, bool UP>
 __device__ __forceinline__ void march_cells(const ProjectArgs& a, const Ray& r, Accumulator<ACC>& acc)
 {
     const char* __restrict__ cells = static_cast<const char*>(a.cells);
@@ -374,6 +401,7 @@ __device__ __forceinline__ void march_cells(const ProjectArgs& a, const Ray& r, 
     const float2 dy2 = make_float2((float)r.step[1], (float)r.step[1]);
     const float2 dz2 = make_float2((float)r.step[2], (float)r.step[2]);
     const uint32_t sy = a.csy, sz = a.csz, cmax = a.cmax, offset = a.coffset;
+    const float up = (float)a.up;
     const float2 two2 = make_float2(2.0f, 2.0f);
     float2 kk = make_float2(0.0f, 1.0f);  // steps k and k + 1
     CellCache cc;
@@ -382,7 +410,7 @@ __device__ __forceinline__ void march_cells(const ProjectArgs& a, const Ray& r, 
         float part = 0.0f;
 #pragma unroll
         for (int j = 0; j < U; j += 2) {
-            const float2 f = cell_sample_pair(cells, kk, fr, dx2, dy2, dz2, sy, sz, cmax, offset, cc);
+            const float2 f = cell_sample_pair<UP>(cells, kk, fr, dx2, dy2, dz2, sy, sz, cmax, offset, up, cc);
             part += f.x;
             part += f.y;
             kk = __fadd2_rn(kk, two2);
@@ -394,13 +422,13 @@ __device__ __forceinline__ void march_cells(const ProjectArgs& a, const Ray& r, 
         // first value of a pair whose second step lies beyond the ray (its cell
         // index is clamped like any other, its value unused)
         for (; k + 1 < r.n; k += 2) {
-            const float2 f = cell_sample_pair(cells, kk, fr, dx2, dy2, dz2, sy, sz, cmax, offset, cc);
+            const float2 f = cell_sample_pair<UP>(cells, kk, fr, dx2, dy2, dz2, sy, sz, cmax, offset, up, cc);
             acc.add(f.x);
             acc.add(f.y);
             kk = __fadd2_rn(kk, two2);
         }
         if (k < r.n)
-            acc.add(cell_sample_pair(cells, kk, fr, dx2, dy2, dz2, sy, sz, cmax, offset, cc).x);
+            acc.add(cell_sample_pair<UP>(cells, kk, fr, dx2, dy2, dz2, sy, sz, cmax, offset, up, cc).x);
     }
 }
 
@@ -720,7 +748,7 @@ __device__ __forceinline__ void march_array(const ProjectArgs& a, const Ray& r, 
     else if (M == Mode::Segments)
         march_segments<ACC, U>(a, r, acc);
     else
-        march_cells<ACC, U>(a, r, acc);
+        march_cells<ACC, U, M == Mode::CellsUp>(a, r, acc);
 }
 
 // The rays of work item `b` for thread `tid`, cell, segment or pair loop (FP32
@@ -761,7 +789,10 @@ __device__ __forceinline__ void cells_item(const ProjectArgs& a, uint32_t b, uin
     store_patch(a, vm, x, y, val, ok);
 }
 
-constexpr int cell_maxreg(Mode m) { return m == Mode::Segments ? CTLCU_SEGMENT_MAXREG : CTLCU_CELL_MAXREG; }
+constexpr int cell_maxreg(Mode m)
+{
+    return m == Mode::Segments || m == Mode::CellsUp ? CTLCU_SEGMENT_MAXREG : CTLCU_CELL_MAXREG;
+}
 
 // Cell, segment or pair loop over one block of the regular grid.
 template <Mode M, Accum ACC, int U>
@@ -920,6 +951,7 @@ cudaError_t launch_acc(const ProjectArgs& a, Mode mode, int dtype, dim3 grid, cu
         return cudaGetLastError();
     case Mode::Cells: return launch_cells<Mode::Cells, ACC>(a, grid, s);
     case Mode::Segments: return launch_cells<Mode::Segments, ACC>(a, grid, s);
+    case Mode::CellsUp: return launch_cells<Mode::CellsUp, ACC>(a, grid, s);
     case Mode::Pairs: return launch_cells<Mode::Pairs, ACC>(a, grid, s);
     }
     return cudaErrorInvalidValue;

@@ -65,7 +65,9 @@ typedef enum {
 
 /*
  * Sample-loop variant.  AUTO picks CELLS for software trilinear interpolation
- * without up-sampling and GATHER otherwise.
+ * without up-sampling and GATHER otherwise; with up-sampling (>= 2) it reads the
+ * cell array in place of the voxels where that array exists or a context without
+ * a memory budget has the room for it.
  *   GATHER  eight scalar loads per sample from the zero-padded voxel array
  *   CELLS   32-byte loads from a derived cell array holding, per trilinear cell,
  *           the 8 coefficients of its interpolation polynomial about the cell

@@ -76,3 +76,43 @@ def test_unusable_matrix_and_partial_warps_leave_the_other_pixels_alone(ctx):
         np.testing.assert_array_equal(out[[0, 2]], good[[0, 2]])
     finally:
         v.release()
+
+
+@pytest.mark.parametrize("shape,voxel", [((1, 1, 1), (24.0, 24.0, 24.0)), ((17, 12, 9), (2.0, 2.5, 3.0)),
+                                         ((33, 5, 40), (1.0, 4.0, 1.0))])
+@pytest.mark.parametrize("factor", [2, 3, 7])
+@pytest.mark.parametrize("storage", [L.F32, L.F16])
+def test_upsampled_volume_read_from_the_cells(ctx, shape, voxel, factor, storage):
+    """Virtual replication through the cell array: against the oracle, and against
+    the gather loop that reads the replicated grid voxel by voxel."""
+    vol = _volume(shape, 7).astype(np.float16).astype(np.float32)  # the same in both storages
+    C, R = 29, 18
+    P = _axis_views(C, R, 1.7, 0.13)
+    for sampling in (0.3, 1.0):
+        st = dict(ray_sampling=sampling, volume_upsampling=factor)
+        want, _ = oracle.project_fp64(vol, voxel, P, C, R, ray_sampling=sampling, upsampling=factor)
+        v = ctx.volume(VoxelVolume(vol, voxel), storage)
+        try:
+            before = v.nbytes
+            gather = ctx.project(v, P, C, R, Settings(kernel=L.KERNEL_GATHER, **st))
+            assert v.nbytes == before
+            got = ctx.project(v, P, C, R, Settings(**st))
+            assert v.nbytes > before  # the cells were built and read
+            assert rel_err(got, want).max() <= 1e-4
+            assert rel_err(gather, want).max() <= 1e-4
+        finally:
+            v.release()
+
+
+def test_upsampled_calls_take_no_array_from_a_memory_budget():
+    """With a budget set the up-sampled call runs as it does without any derived array."""
+    vol = _volume((20, 20, 20), 9)
+    P = _axis_views(16, 16, 4.0, 0.1)
+    with Context(0) as c:
+        v = c.volume(VoxelVolume(vol, (1.0, 1.0, 1.0)))
+        want = c.project(v, P, 16, 16, Settings(volume_upsampling=2, kernel=L.KERNEL_GATHER))
+        used = c.memory_used()
+        c.set_memory_budget(used + 1000)
+        got = c.project(v, P, 16, 16, Settings(volume_upsampling=2))
+        assert c.memory_used() == used
+        np.testing.assert_array_equal(got, want)
