@@ -583,6 +583,9 @@ int volume_args(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, Project
     for (int k = 0; k < 3; ++k) {
         a.voxel[k] = (double)voxel[k];
         a.corner[k] = (double)d.offset_mm[k] - 0.5 * (double)a.grid[k] * a.voxel[k];
+        a.scale[k] = a.increment / a.voxel[k];
+        a.inv_voxel[k] = 1.0 / a.voxel[k];
+        a.corner_v[k] = a.corner[k] / a.voxel[k];
     }
     return CTLCU_OK;
 }

@@ -184,6 +184,9 @@ struct ProjectArgs {
     double voxel[3];          // voxel size of that grid (mm)
     double corner[3];         // low corner of that grid (mm)
     double increment;         // step length (mm)
+    double scale[3];          // increment / voxel
+    double inv_voxel[3];      // 1 / voxel
+    double corner_v[3];       // corner / voxel
     const void* cells;        // Mode::Cells, Segments and CellsUp: coefficient cells; Mode::Pairs: pair entries
     uint32_t csy, csz;        // their strides (CellLayout, PairLayout)
     uint32_t cmax;            // last valid index
