@@ -291,7 +291,6 @@ int make_volume(ctlcu_ctx* ctx, const ctlcu_volume_desc* d, const float* data, b
         CU_TRY(ctx, cudaMallocAsync(&v.data, bytes, ctx->stream));
     else
         CU_TRY(ctx, cudaMalloc(&v.data, bytes));
-    CU_TRY(ctx, cudaMemsetAsync(v.data, 0, bytes, ctx->stream));
     const size_t nbytes = (size_t)n[0] * n[1] * n[2] * sizeof(float);
     const float* src = data;
     float* staging = nullptr;

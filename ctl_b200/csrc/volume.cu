@@ -8,6 +8,8 @@
 // math in raycast.cu) and materialised only for the hardware-texture path.
 #include "internal.cuh"
 
+#include <algorithm>
+
 namespace ctlcu {
 
 namespace {
@@ -30,21 +32,25 @@ __device__ __forceinline__ float to_float<__nv_bfloat16>(__nv_bfloat16 v) { retu
 template <>
 __device__ __forceinline__ float to_float<__half>(__half v) { return __half2float(v); }
 
-// dst (padded, zero-initialised by the caller) <- convert(src), one thread per voxel
+// dst (padded) <- convert(src), borders zero: a warp per row of the padded array, so
+// that every element is written once and only a row's place takes a division.
+// 256^3 FP32: 73 us for a memset and one thread per voxel, 23 us now.
 template <typename T>
-__global__ void pad_convert_kernel(const float* __restrict__ src, T* __restrict__ dst, int nx, int ny,
-                                   int nz)
+__global__ void __launch_bounds__(256)
+    pad_convert_kernel(const float* __restrict__ src, T* __restrict__ dst, int nx, int ny, int nz)
 {
-    const int ex = nx + 2 * kPad, ey = ny + 2 * kPad;
-    const size_t total = (size_t)nx * ny * nz;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
-         i += (size_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i % nx);
-        const size_t r = i / nx;
-        const int y = (int)(r % ny);
-        const int z = (int)(r / ny);
-        dst[(size_t)(x + kPad) + (size_t)ex * ((size_t)(y + kPad) + (size_t)ey * (size_t)(z + kPad))] =
-            from_float<T>(src[i]);
+    const int ex = nx + 2 * kPad, ey = ny + 2 * kPad, ez = nz + 2 * kPad;
+    const uint32_t rows = (uint32_t)ey * (uint32_t)ez, lane = threadIdx.x & 31u;
+    for (uint32_t r = blockIdx.x * 8u + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8u) {
+        const int z = (int)(r / (uint32_t)ey) - kPad, y = (int)(r % (uint32_t)ey) - kPad;
+        const bool inside = z >= 0 && z < nz && y >= 0 && y < ny;
+        const float* from = src + ((size_t)z * ny + y) * nx - kPad;
+        T* to = dst + (size_t)r * ex;
+#pragma unroll 4
+        for (int x = (int)lane; x < ex; x += 32) {
+            const bool in = inside && x >= kPad && x < nx + kPad;
+            to[x] = from_float<T>(in ? __ldg(from + x) : 0.0f);
+        }
     }
 }
 
@@ -113,43 +119,68 @@ __global__ void upsample_kernel(const T* __restrict__ padded, int nx, int ny, in
 // coefficients are computed in FP64 and stored as FP32 in the order
 //   (C0, Cz), (Cx, Cxz), (Cy, Cyz), (Cxy, Cxyz)
 // so the sampler evaluates f with three packed f32x2 FMAs and one FMA.
-template <typename T>
-__global__ void build_cells_kernel(const T* __restrict__ padded, int ex, int ey, int ez, uint32_t csy,
-                                   uint32_t csz, float4* __restrict__ cells)
+//
+// Bound by writing the cells (32 bytes each) once.  A thread writes the slots of
+// one place in the rows of a slice pair (CellLayout: lanes alternate between the two
+// slices, so a warp writes 1 KB runs), `per` rows one after the other, and keeps the z and x sums and
+// differences of the previous row: four voxel loads, four conversions and 20 FP64
+// additions per cell.  Slots beyond the last cell of a row, a pair or an odd last
+// slice are written as zeros.  256^3 FP32: 240 us with 64 FP64 operations per cell
+// and a memset of the array before, 123 us now (4.8 TB/s).
+__device__ __forceinline__ void store_cell(float* p, float4 lo, float4 hi)
 {
-    const int cx = ex - 1, cy = ey - 1, cz = ez - 1;
-    const size_t total = (size_t)cx * cy * cz;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
-         i += (size_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i % cx);
-        const size_t r = i / cx;
-        const int y = (int)(r % cy);
-        const int z = (int)(r / cy);
-        const size_t o = (size_t)x + (size_t)ex * ((size_t)y + (size_t)ey * z);
-        const size_t sy = ex, sz = (size_t)ex * ey;
-        double v[2][2][2];  // [z][y][x]
-        for (int c = 0; c < 2; ++c)
-            for (int b = 0; b < 2; ++b)
-                for (int a = 0; a < 2; ++a)
-                    v[c][b][a] = (double)to_float<T>(padded[o + a + b * sy + c * sz]);
-        double C0 = 0, Cx = 0, Cy = 0, Cz = 0, Cxy = 0, Cxz = 0, Cyz = 0, Cxyz = 0;
-        for (int c = 0; c < 2; ++c)
-            for (int b = 0; b < 2; ++b)
-                for (int a = 0; a < 2; ++a) {
-                    const double sx = a ? 1.0 : -1.0, sy_ = b ? 1.0 : -1.0, sz_ = c ? 1.0 : -1.0;
-                    const double t = v[c][b][a];
-                    C0 += t;
-                    Cx += sx * t;
-                    Cy += sy_ * t;
-                    Cz += sz_ * t;
-                    Cxy += sx * sy_ * t;
-                    Cxz += sx * sz_ * t;
-                    Cyz += sy_ * sz_ * t;
-                    Cxyz += sx * sy_ * sz_ * t;
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 :: "l"(p), "f"(lo.x), "f"(lo.y), "f"(lo.z), "f"(lo.w), "f"(hi.x), "f"(hi.y), "f"(hi.z), "f"(hi.w)
+                 : "memory");
+}
+
+template <typename T>
+__global__ void __launch_bounds__(128)
+    build_cells_kernel(const T* __restrict__ padded, int ex, int ey, CellLayout L, uint32_t per,
+                       float* __restrict__ cells)
+{
+    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t pairs = (L.cz + 1) / 2;
+    const uint32_t rows = (L.sz + L.sy - 1) / L.sy;  // the last one may be the pair's tail alone
+    if (slot >= L.sy)
+        return;
+    const uint32_t x = slot >> 1;
+    const size_t ys = (size_t)ex, zs = (size_t)ex * ey;
+    for (uint32_t p = blockIdx.z; p < pairs; p += gridDim.z) {
+        const uint32_t z = 2 * p + (slot & 1u);
+        const bool column = x < L.cx && z < L.cz;
+        for (uint32_t y0 = blockIdx.y * per; y0 < rows; y0 += gridDim.y * per) {
+            const uint32_t y1 = min(y0 + per, rows);
+            const T* v = padded + (x + ys * y0 + zs * z);
+            // sums and differences over x, z of one row: s, sx (x), sz (z), sxz
+            double s = 0.0, sx = 0.0, sz = 0.0, sxz = 0.0;
+            auto row = [&]() {
+                const double a = to_float<T>(v[0]), b = to_float<T>(v[1]);
+                const double c = to_float<T>(v[zs]), d = to_float<T>(v[zs + 1]);
+                const double l = a + b, lx = b - a, h = c + d, hx = d - c;
+                s = l + h;
+                sx = lx + hx;
+                sz = h - l;
+                sxz = hx - lx;
+            };
+            if (column && y0 < L.cy)
+                row();
+            for (uint32_t y = y0; y < y1; ++y) {
+                const size_t i = (size_t)p * L.sz + (size_t)y * L.sy + slot;
+                float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+                if (column && y < L.cy) {
+                    const double s0 = s, x0 = sx, z0 = sz, xz0 = sxz;
+                    v += ys;
+                    row();
+                    lo = make_float4((float)((s0 + s) * 0.125), (float)((z0 + sz) * 0.25), (float)((x0 + sx) * 0.25),
+                                     (float)((xz0 + sxz) * 0.5));
+                    hi = make_float4((float)((s - s0) * 0.25), (float)((sz - z0) * 0.5), (float)((sx - x0) * 0.5),
+                                     (float)(sxz - xz0));
                 }
-        const size_t c = cell_linear((uint32_t)x, (uint32_t)y, (uint32_t)z, csy, csz, 0u);
-        cells[2 * c] = make_float4((float)(C0 * 0.125), (float)(Cz * 0.25), (float)(Cx * 0.25), (float)(Cxz * 0.5));
-        cells[2 * c + 1] = make_float4((float)(Cy * 0.25), (float)(Cyz * 0.5), (float)(Cxy * 0.5), (float)Cxyz);
+                if (i < (size_t)(p + 1) * L.sz)
+                    store_cell(cells + 8 * i, lo, hi);
+            }
+        }
     }
 }
 
@@ -184,7 +215,8 @@ unsigned grid_for(size_t n)
 
 cudaError_t launch_pad_convert(const float* src, void* dst, const int n[3], int dtype, cudaStream_t s)
 {
-    const unsigned g = grid_for((size_t)n[0] * n[1] * n[2]);
+    const uint32_t rows = (uint32_t)(n[1] + 2 * kPad) * (uint32_t)(n[2] + 2 * kPad);
+    const unsigned g = std::min<uint32_t>((rows + 7) / 8, 148u * 32u);
     switch (dtype) {
     case 0: pad_convert_kernel<float><<<g, 256, 0, s>>>(src, (float*)dst, n[0], n[1], n[2]); break;
     case 1: pad_convert_kernel<__nv_bfloat16><<<g, 256, 0, s>>>(src, (__nv_bfloat16*)dst, n[0], n[1], n[2]); break;
@@ -215,16 +247,18 @@ cudaError_t launch_mean_volume(const double* sum, double count, float* dst_padde
 cudaError_t launch_build_cells(const void* padded, const int n[3], int dtype, const CellLayout& L,
                                void* cells, cudaStream_t s)
 {
-    const int ex = n[0] + 2 * kPad, ey = n[1] + 2 * kPad, ez = n[2] + 2 * kPad;
-    const unsigned g = grid_for((size_t)(ex - 1) * (ey - 1) * (ez - 1));
-    // the stride padding between slices is never sampled; keep it zero
-    cudaError_t e = cudaMemsetAsync(cells, 0, L.count * kCellBytes, s);
-    if (e != cudaSuccess)
-        return e;
+    const int ex = n[0] + 2 * kPad, ey = n[1] + 2 * kPad;
+    // rows per thread: 16 where that leaves enough blocks to fill the GPU, fewer for
+    // small volumes (64^3: 17 us with 16 rows, 7.4 with 2)
+    const uint32_t rows = (L.sz + L.sy - 1) / L.sy, pairs = (L.cz + 1) / 2, bx = (L.sy + 127) / 128;
+    uint32_t per = 16;
+    while (per > 1 && (uint64_t)bx * ((rows + per - 1) / per) * pairs < 148u * 12u)
+        per /= 2;
+    const dim3 g(bx, std::min<uint32_t>((rows + per - 1) / per, 65535u), std::min<uint32_t>(pairs, 65535u));
     switch (dtype) {
-    case 0: build_cells_kernel<float><<<g, 256, 0, s>>>((const float*)padded, ex, ey, ez, L.sy, L.sz, (float4*)cells); break;
-    case 1: build_cells_kernel<__nv_bfloat16><<<g, 256, 0, s>>>((const __nv_bfloat16*)padded, ex, ey, ez, L.sy, L.sz, (float4*)cells); break;
-    case 2: build_cells_kernel<__half><<<g, 256, 0, s>>>((const __half*)padded, ex, ey, ez, L.sy, L.sz, (float4*)cells); break;
+    case 0: build_cells_kernel<float><<<g, 128, 0, s>>>((const float*)padded, ex, ey, L, per, (float*)cells); break;
+    case 1: build_cells_kernel<__nv_bfloat16><<<g, 128, 0, s>>>((const __nv_bfloat16*)padded, ex, ey, L, per, (float*)cells); break;
+    case 2: build_cells_kernel<__half><<<g, 128, 0, s>>>((const __half*)padded, ex, ey, L, per, (float*)cells); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
