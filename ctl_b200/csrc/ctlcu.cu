@@ -375,7 +375,7 @@ int ensure_cells(ctlcu_ctx* ctx, VolumeEntry& v)
         return CTLCU_OK;
     const int n[3] = { (int)v.desc.n[0], (int)v.desc.n[1], (int)v.desc.n[2] };
     const CellLayout L = cell_layout(n);
-    const size_t bytes = (size_t)L.count * kCellBytes;
+    const size_t bytes = (size_t)L.count * kCellBytes + kSupportBytes;
     if (ctx->budget && ctx->used + bytes > ctx->budget)
         return fail(ctx, CTLCU_ERR_OUT_OF_MEMORY,
                     "cell array of %zu bytes exceeds the memory budget (%llu of %llu bytes used)", bytes,
@@ -574,7 +574,9 @@ int volume_args(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, Project
         a.csz = L.sz;
         a.cmax = L.max_index;
         a.coffset = L.offset;
+        a.support = cell_support(v.cells, L);
     }
+    a.dtype = dtype;
     a.sy = a.ext[0];
     a.sz = a.ext[0] * a.ext[1];
     const float smallest = std::min(std::min(voxel[0], voxel[1]), voxel[2]);

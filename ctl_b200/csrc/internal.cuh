@@ -140,6 +140,23 @@ inline CellLayout cell_layout(const int n[3])
     return L;
 }
 
+// Bounds of the cells whose eight voxels are not all zero, behind the last cell: the
+// maxima over them of -x, x, -y, y, -z, z, -(x+y), x+y, -(x-y), x-y (cell indexes), or
+// kSupportNone; then kSupportNone, or 1 where a voxel is infinite or not a number.  Air around the object and the corners outside a scanner's circular
+// field of view are exact zeros; a ray's samples there add nothing, so the cell
+// loops start and end at these slabs (the diagonal pairs make the outline an
+// octagon).  With cylinders of 90% of the volume's width: 256^3 -> 60 x 512^2 11.2 ->
+// 9.1 ms, 512^3 helical, 180 views, 2.15 -> 1.54 ms; volumes without zeros: 11.2 ->
+// 11.4 and 2.14 -> 2.17 ms.
+constexpr int kSupport = 11, kSupportNonFinite = 10;
+constexpr size_t kSupportBytes = 64;
+constexpr int kSupportNone = (int)0x80808080;  // a byte pattern: set by memset
+
+inline int* cell_support(void* cells, const CellLayout& L)
+{
+    return reinterpret_cast<int*>(static_cast<char*>(cells) + L.count * kCellBytes);
+}
+
 // x-pair array: for every padded voxel (x < ext_x - 1, y, z) the float2
 // (mid, diff) = ((v[x] + v[x+1]) / 2, v[x+1] - v[x]), computed in FP64.  A
 // trilinear cell reads four entries (its two rows in y times two slices in
@@ -181,6 +198,7 @@ struct ProjectArgs {
     int sy, sz;               // padded strides (voxels)
     int grid[3];              // voxel grid the rays see (f * n, or 1 for the mean voxel)
     int up;                   // virtual up-sampling factor (>= 1)
+    int dtype;                // storage of vol (ctlcu_dtype)
     double voxel[3];          // voxel size of that grid (mm)
     double corner[3];         // low corner of that grid (mm)
     double increment;         // step length (mm)
@@ -191,6 +209,7 @@ struct ProjectArgs {
     uint32_t csy, csz;        // their strides (CellLayout, PairLayout)
     uint32_t cmax;            // last valid index
     uint32_t coffset;         // CellLayout::offset
+    const int* support;       // kSupport bounds of the cells that are not zero
     uint32_t vm_group;        // view groups per chunk of the block order
     uint32_t n_views;         // views (n_vm / n_modules)
     uint32_t view_groups;     // ceil(n_views / views per block)

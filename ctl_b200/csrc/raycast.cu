@@ -199,6 +199,27 @@ __device__ __forceinline__ Ray setup_ray_cells(const ProjectArgs& a, const ViewG
         far = fmin(far, fmax(l1, l2));
     }
     const double t0 = fmax(near, 0.0);
+    double first = t0, last = far;  // of the samples that are not zero
+    if (M != Mode::Pairs) {
+        // clipped to the slabs of the cells that are not zero, a thousandth of a voxel
+        // wider for the FP32 positions; cell i covers i - 1/2 .. i + 1/2 in v
+        const double f = M == Mode::CellsUp ? (double)a.up : 1.0;
+        const double dir[5] = { d[0], d[1], d[2], d[0] + d[1], d[0] - d[1] };
+        const double pos[5] = { s[0], s[1], s[2], s[0] + s[1], s[0] - s[1] };
+        const double wide[5] = { 0.501, 0.501, 0.501, 1.002, 1.002 };
+        const double shift[5] = { 1.0 - kPad, 1.0 - kPad, 1.0 - kPad, 2.0 - 2 * kPad, 0.0 };
+        for (int i = 0; i < 5; ++i) {
+            const double lo = f * (shift[i] - wide[i] - __ldg(a.support + 2 * i));
+            const double hi = f * (shift[i] + wide[i] + __ldg(a.support + 2 * i + 1));
+            // a diagonal's reciprocal from FP32 and one Newton step (4e-15), well within
+            // the margin; where FP32 cannot hold it, it is NaN and the slab is passed over
+            const double r0 = __frcp_rn((float)dir[i]);
+            const double inv = i < 3 ? 1.0 / dir[i] : r0 * fma(-dir[i], r0, 2.0);
+            const double l1 = (lo - pos[i]) * inv, l2 = (hi - pos[i]) * inv;
+            first = fmax(first, fmin(l1, l2));
+            last = fmin(last, fmax(l1, l2));
+        }
+    }
     // a ray that misses, or whose direction is not a number
     const bool hit = near <= far && far >= 0.0 && rn * 0.0 == 0.0;
     // the box diagonal bounds any honest ray; beyond it the inputs are broken
@@ -206,7 +227,7 @@ __device__ __forceinline__ Ray setup_ray_cells(const ProjectArgs& a, const ViewG
         if (flags)
             atomicOr(flags, kFlagNonFinite);
     } else if (hit) {
-        const double i0 = ceil(t0), i1 = floor(far);
+        const double i0 = ceil(first), i1 = floor(last);
         r.n = i1 >= i0 ? static_cast<int>(i1 - i0) + 1 : 0;
         r.first = static_cast<int>(fmin(i0, 1.0e9));
         for (int i = 0; i < 3; ++i) {
@@ -862,6 +883,24 @@ __device__ __forceinline__ void store_patch(const ProjectArgs& a, uint32_t vm, u
     }
 }
 
+// One ray of the gather loop, up-sampled.  A voxel that is infinite or not a number
+// reaches a whole cell through the cell's polynomial, where the replicated grid holds
+// it to the samples next to that voxel: volumes with such voxels take this road.
+template <Accum ACC>
+__device__ __noinline__ void gather_upsampled(const ProjectArgs& a, const ViewGeom& g, double px, double py, bool live,
+                                              Accumulator<ACC>& acc)
+{
+    if (!live)
+        return;
+    const Ray r = setup_ray<Mode::Trilinear>(a, g, px, py, a.flags);
+    if (a.dtype == 0)
+        march_trilinear<float, ACC, true>(a, r, acc);
+    else if (a.dtype == 1)
+        march_trilinear<__nv_bfloat16, ACC, true>(a, r, acc);
+    else
+        march_trilinear<__half, ACC, true>(a, r, acc);
+}
+
 // The sample loop of a derived array's mode.
 template <Mode M, Accum ACC, int U>
 __device__ __forceinline__ void march_array(const ProjectArgs& a, const Ray& r, Accumulator<ACC>& acc)
@@ -886,7 +925,13 @@ __device__ __forceinline__ void cells_item(const ProjectArgs& a, uint32_t b, uin
     const ViewGeom& g = a.geom[ok ? vm : 0u];
     const bool live = ok && g.valid;
     Accumulator<ACC> acc;
-    if (a.rays_x == 1 && a.rays_y == 1) {
+    if (M == Mode::CellsUp && __ldg(a.support + kSupportNonFinite) > 0) {
+        const double ix = 1.0 / a.rays_x, iy = 1.0 / a.rays_y;
+        for (uint32_t rx = 0; rx < a.rays_x; ++rx)
+            for (uint32_t ry = 0; ry < a.rays_y; ++ry)
+                gather_upsampled<ACC>(a, g, (double)x - 0.5 + 0.5 * ix + rx * ix, (double)y - 0.5 + 0.5 * iy + ry * iy,
+                                      live, acc);
+    } else if (a.rays_x == 1 && a.rays_y == 1) {
         // one ray through the pixel centre (x - 0.5 + 0.5 is x exactly): the
         // pixel and its geometry are dead once the ray is set up, so the
         // sample loop carries only the ray
@@ -919,7 +964,7 @@ constexpr int cell_maxreg(Mode m)
 
 // Cell, segment or pair loop over one block of the regular grid.
 template <Mode M, Accum ACC, int U>
-__global__ void __maxnreg__(cell_maxreg(M)) cells_kernel(const ProjectArgs a)
+__global__ void __maxnreg__(cell_maxreg(M)) cells_kernel(const __grid_constant__ ProjectArgs a)
 {
     cells_item<M, ACC, U>(a, blockIdx.x, threadIdx.x);
 }
@@ -973,7 +1018,7 @@ __global__ void __maxnreg__(cell_maxreg(M))
 
 // Gather, nearest-voxel and texture loops over one block of the regular grid.
 template <typename T, Mode M, Accum ACC, bool UP>
-__global__ void __maxnreg__(CTLCU_GATHER_MAXREG) project_kernel(const ProjectArgs a)
+__global__ void __maxnreg__(CTLCU_GATHER_MAXREG) project_kernel(const __grid_constant__ ProjectArgs a)
 {
     static_assert(M == Mode::Trilinear || M == Mode::Nearest || M == Mode::Texture, "cells_kernel runs these");
     uint32_t vm, x, y;

@@ -146,3 +146,36 @@ def test_nearest_voxel_sums_match_the_oracle(ctx, shape, voxel, sampling, tilt):
             assert rel_err(got, want)[~ties].max() <= 1e-4
     finally:
         v.release()
+
+
+@pytest.mark.parametrize("where", ["one voxel", "corner block", "diagonal", "empty", "nan"])
+@pytest.mark.parametrize("upsampling", [1, 3])
+@pytest.mark.parametrize("sampling", [0.3, 1.0])
+def test_zero_voxels_outside_the_object_change_nothing(ctx, where, upsampling, sampling):
+    """The loops start and end at the bounds of the voxels that are not zero: single
+    voxels, blocks at a corner, along a diagonal, nothing at all, and a NaN."""
+    n = (27, 22, 31)
+    vol = np.zeros(n[::-1], np.float32)
+    if where == "one voxel":
+        vol[13, 0, 26] = 0.04
+    elif where == "corner block":
+        vol[25:, 17:, :6] = _volume((6, 5, 6), 3)
+    elif where == "diagonal":
+        for i in range(22):
+            vol[i, i, 21 - i] = 0.03
+    elif where == "nan":
+        vol[4, 5, 6] = np.nan
+    C, R = 45, 37
+    P = np.concatenate([_axis_views(C, R, 1.5, t) for t in (0.0, 0.21, 1.0)])
+    got = ctx.project_volume(VoxelVolume(vol, (1.0, 1.2, 0.9)), P, C, R,
+                             Settings(ray_sampling=sampling, volume_upsampling=upsampling))
+    if where == "empty":
+        np.testing.assert_array_equal(got, 0.0)
+        return
+    if where == "nan":  # seen by the rays that pass it, and by no others
+        seen, _ = oracle.project_fp64(np.nan_to_num(vol, nan=1.0), (1.0, 1.2, 0.9), P, C, R, ray_sampling=sampling,
+                                      upsampling=upsampling)
+        assert np.isnan(got[seen > 1e-3]).all() and not np.isnan(got[seen == 0]).any() and (seen > 1e-3).any()
+        return
+    want, _ = oracle.project_fp64(vol, (1.0, 1.2, 0.9), P, C, R, ray_sampling=sampling, upsampling=upsampling)
+    assert want.max() > 0 and rel_err(got, want).max() <= 1e-4
