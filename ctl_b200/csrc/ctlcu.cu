@@ -69,6 +69,7 @@ struct ctlcu_ctx {
         LaunchShape shape;
     };
     std::map<std::tuple<uint64_t, uint32_t, uint32_t, uint32_t>, Tuned> tuned;
+    HostCopier copier;  // threads' pinned slots for pageable host memory, allocated on first use
     DenStaging den;  // pinned buffers for DEN file streaming, allocated on first use
     cudaStream_t copy_stream = nullptr;  // device-to-host copies that overlap projection
     cudaStream_t aux_stream = nullptr;   // every other chunk of a projection into host memory
@@ -132,6 +133,17 @@ Mem mem_kind(const void* p)
         return Mem::Foreign;
     }
     return attr.device == cur ? Mem::Local : Mem::Foreign;
+}
+
+// Host memory the driver does not know (neither pinned nor managed).
+bool pageable(const void* p)
+{
+    cudaPointerAttributes attr;
+    if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return attr.type == cudaMemoryTypeUnregistered;
 }
 
 // Device memory of the current device (see mem_kind).  Memory of another GPU
@@ -296,7 +308,11 @@ int make_volume(ctlcu_ctx* ctx, const ctlcu_volume_desc* d, const float* data, b
     float* staging = nullptr;
     if (!on_device) {
         CU_TRY(ctx, cudaMallocAsync((void**)&staging, nbytes, ctx->stream));
-        CU_TRY(ctx, cudaMemcpyAsync(staging, data, nbytes, cudaMemcpyHostToDevice, ctx->stream));
+        if (nbytes >= HostCopier::kLeast && pageable(data) && ctx->copier.ensure() == cudaSuccess)
+            CU_TRY(ctx, ctx->copier.run(ctx->device, { { staging, const_cast<float*>(data), nbytes, nullptr } }, false,
+                                        ctx->stream));
+        else
+            CU_TRY(ctx, cudaMemcpyAsync(staging, data, nbytes, cudaMemcpyHostToDevice, ctx->stream));
         src = staging;
     }
     CU_TRY(ctx, launch_pad_convert(src, v.data, n, d->dtype, ctx->stream));
@@ -760,6 +776,11 @@ int project_any(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, const d
         // alternate between two streams, so that a chunk's first blocks fill
         // the SMs that the previous chunk's last blocks leave idle, and the
         // last chunks are small, so that little copying follows the last kernel.
+        // A copy into pageable memory returns only when it is done: all chunks are
+        // launched first and several threads copy behind them (a 256^3 host volume,
+        // 30 x 512^2 into host memory: 14.0 -> 7.7 ms, with the upload's threads).
+        const bool threads = out_bytes >= HostCopier::kLeast && pageable(out) && ctx->copier.ensure() == cudaSuccess;
+        std::vector<HostCopyPart> parts;
         if (!ctx->copy_stream)
             CU_TRY(ctx, cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
         if (!ctx->aux_stream)
@@ -788,6 +809,11 @@ int project_any(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, const d
             cudaError_t e = r ? cudaSuccess : cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
             if (!r && e == cudaSuccess)
                 e = cudaEventRecord(done, cs);
+            if (!r && e == cudaSuccess && threads) {
+                parts.push_back({ d_out + first * view_values, out + first * view_values,
+                                  sizeof(float) * n * view_values, done });
+                continue;
+            }
             if (!r && e == cudaSuccess)
                 e = cudaStreamWaitEvent(ctx->copy_stream, done, 0);
             if (!r && e == cudaSuccess)
@@ -798,6 +824,13 @@ int project_any(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, const d
             if (!r && e != cudaSuccess)
                 r = fail(ctx, CTLCU_ERR_CUDA, "copy of projections to the host failed: %s", cudaGetErrorString(e));
         }
+        if (!parts.empty() && r == CTLCU_OK) {
+            const cudaError_t e = ctx->copier.run(ctx->device, parts, true, ctx->copy_stream);
+            if (e != cudaSuccess)
+                r = fail(ctx, CTLCU_ERR_CUDA, "copy of projections to the host failed: %s", cudaGetErrorString(e));
+        }
+        for (HostCopyPart& p : parts)
+            cudaEventDestroy(p.after);
         // the device buffers are freed on `st`: order that after the last copy
         // and after everything on the second stream
         cudaEvent_t copied = nullptr, aux_done = nullptr;
@@ -1304,6 +1337,7 @@ int ctlcu_destroy(ctlcu_ctx* ctx)
         if (ctx->order)
             cudaEventDestroy(ctx->order);
         ctx->den.release();
+        ctx->copier.release();
         if (ctx->copy_stream) {
             cudaStreamSynchronize(ctx->copy_stream);
             cudaStreamDestroy(ctx->copy_stream);

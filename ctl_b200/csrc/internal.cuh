@@ -304,6 +304,7 @@ cudaError_t launch_transform(float* data, uint64_t per_view, uint32_t n_views, c
 
 #include <cstdio>
 #include <string>
+#include <vector>
 
 #include <nvtx3/nvToolsExt.h>
 
@@ -325,6 +326,29 @@ struct DenStaging {
     cudaEvent_t ev[2] = { nullptr, nullptr };
     cudaError_t ensure();
     void release();
+};
+// Copies between pageable host memory and the device by several threads through pinned
+// slots (hostcopy.cu); a context keeps one, allocated on first use: at most 8 threads'
+// slots, 32 MB.
+struct HostCopyPart {
+    void* device;
+    void* host;         // read only when copying to the device
+    size_t bytes;
+    cudaEvent_t after;  // event the copy waits for, or null
+};
+struct HostCopier {
+    static constexpr size_t kSlot = 2u << 20;
+    static constexpr int kMaxWorkers = 8;
+    // from here on the threads' start costs less than they save
+    static constexpr size_t kLeast = 8u << 20;
+    void* base = nullptr;
+    cudaEvent_t ev[2 * kMaxWorkers] = {};
+    int workers = 0;
+    bool ready = false;
+    char* slot(int i) { return static_cast<char*>(base) + kSlot * (size_t)i; }
+    cudaError_t ensure();
+    void release();
+    cudaError_t run(int device, const std::vector<HostCopyPart>& parts, bool to_host, cudaStream_t st);
 };
 int den_write(const char* path, const void* data, uint32_t elem, uint32_t rows, uint32_t cols, uint32_t count,
               cudaStream_t st, DenStaging* stage, std::string& msg);
