@@ -228,6 +228,8 @@ struct ProjectArgs {
     uint32_t n_modules;
     uint32_t tiles_x, tiles_per_vm;
     uint32_t rays_x, rays_y;
+    uint32_t sub_x, sub_y;    // log2 of rays_x, rays_y where each sub-ray has a lane, else 0
+    uint32_t span_x, span_y;  // channels << sub_x, rows << sub_y
     int* flags;
     unsigned long long* counter;  // sample count (count kernel only)
 };

@@ -809,7 +809,8 @@ __device__ __forceinline__ void march_texture(const ProjectArgs& a, const Ray& r
     }
 }
 
-// Pixel of thread `tid` of work item (block) `b` of a.block threads, for the
+// Pixel (with sub-rays spread over lanes, sub-ray of the finer grid of channels <<
+// sub_x by rows << sub_y) of thread `tid` of work item (block) `b` of a.block threads, for the
 // launch shape in `a` (every factor of the mapping is a power of two).
 __device__ __forceinline__ bool pixel_of_item(const ProjectArgs& a, uint32_t b, uint32_t tid, uint32_t& vm,
                                               uint32_t& x, uint32_t& y)
@@ -839,7 +840,7 @@ __device__ __forceinline__ bool pixel_of_item(const ProjectArgs& a, uint32_t b, 
     const uint32_t ly_shift = 5u - a.lx_shift;
     x = (tx << a.tx_shift) + ((w & ((1u << a.wx_shift) - 1u)) << a.lx_shift) + (lane >> ly_shift);
     y = (ty << a.ty_shift) + ((w >> a.wx_shift) << ly_shift) + (lane & ((1u << ly_shift) - 1u));
-    return view < a.n_views && x < a.channels && y < a.rows;
+    return view < a.n_views && x < a.span_x && y < a.span_y;
 }
 
 __device__ __forceinline__ bool pixel_of_thread(const ProjectArgs& a, uint32_t tid, uint32_t& vm, uint32_t& x,
@@ -925,36 +926,51 @@ __device__ __forceinline__ void cells_item(const ProjectArgs& a, uint32_t b, uin
     const ViewGeom& g = a.geom[ok ? vm : 0u];
     const bool live = ok && g.valid;
     Accumulator<ACC> acc;
-    if (M == Mode::CellsUp && __ldg(a.support + kSupportNonFinite) > 0) {
-        const double ix = 1.0 / a.rays_x, iy = 1.0 / a.rays_y;
-        for (uint32_t rx = 0; rx < a.rays_x; ++rx)
-            for (uint32_t ry = 0; ry < a.rays_y; ++ry)
-                gather_upsampled<ACC>(a, g, (double)x - 0.5 + 0.5 * ix + rx * ix, (double)y - 0.5 + 0.5 * iy + ry * iy,
-                                      live, acc);
-    } else if (a.rays_x == 1 && a.rays_y == 1) {
-        // one ray through the pixel centre (x - 0.5 + 0.5 is x exactly): the
-        // pixel and its geometry are dead once the ray is set up, so the
-        // sample loop carries only the ray
-        Ray r = setup_ray_cells<M>(a, g, (double)x, (double)y, live ? a.flags : nullptr);
+    // (up-sampled volumes with voxels that are no numbers, see gather_upsampled)
+    const bool by_voxel = M == Mode::CellsUp && __ldg(a.support + kSupportNonFinite) > 0;
+    auto ray = [&](double px, double py) {
+        if (by_voxel) {
+            gather_upsampled<ACC>(a, g, px, py, live, acc);
+            return;
+        }
+        Ray r = setup_ray_cells<M>(a, g, px, py, live ? a.flags : nullptr);
         if (!live)
             r.n = 0;
         march_array<M, ACC, U>(a, r, acc);
-    } else {
-        const double ix = 1.0 / a.rays_x, iy = 1.0 / a.rays_y;
-        for (uint32_t rx = 0; rx < a.rays_x; ++rx)
-            for (uint32_t ry = 0; ry < a.rays_y; ++ry) {
-                const double px = (double)x - 0.5 + 0.5 * ix + rx * ix;
-                const double py = (double)y - 0.5 + 0.5 * iy + ry * iy;
-                Ray r = setup_ray_cells<M>(a, g, px, py, live ? a.flags : nullptr);
-                if (!live)
-                    r.n = 0;
-                march_array<M, ACC, U>(a, r, acc);
-            }
+    };
+    if (a.rays_x == 1 && a.rays_y == 1) {
+        // one ray through the pixel centre (x - 0.5 + 0.5 is x exactly): the
+        // pixel and its geometry are dead once the ray is set up, so the
+        // sample loop carries only the ray
+        ray((double)x, (double)y);
+        const float val = static_cast<float>(a.increment * acc.value());
+        // the pixel again for the store, rather than holding it through the loop
+        pixel_of_item(a, b, tid, vm, x, y);
+        store_patch(a, vm, x, y, val, ok);
+        return;
     }
-    const float val = static_cast<float>(a.increment * acc.value() / (double)(a.rays_x * a.rays_y));
-    // the pixel again for the store, rather than holding it through the loop
+    const bool spread = (a.sub_x | a.sub_y) != 0;  // a lane per sub-ray
+    const double ix = 1.0 / a.rays_x, iy = 1.0 / a.rays_y;
+    const uint32_t nx = spread ? 1u : a.rays_x, ny = spread ? 1u : a.rays_y;
+    const uint32_t x0 = spread ? x & (a.rays_x - 1u) : 0u, y0 = spread ? y & (a.rays_y - 1u) : 0u;
+    for (uint32_t rx = 0; rx < nx; ++rx)
+        for (uint32_t ry = 0; ry < ny; ++ry)
+            ray((double)(x >> a.sub_x) - 0.5 + 0.5 * ix + (x0 + rx) * ix,
+                (double)(y >> a.sub_y) - 0.5 + 0.5 * iy + (y0 + ry) * iy);
+    double sum = acc.value();
+    if (spread) {
+        const uint32_t ls = 5u - a.lx_shift;  // log2 of the patch height
+        for (uint32_t o = 1; o < a.rays_y; o <<= 1)
+            sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        for (uint32_t o = 1; o < a.rays_x; o <<= 1)
+            sum += __shfl_xor_sync(0xffffffffu, sum, o << ls);
+    }
+    const float val = static_cast<float>(a.increment * sum / (double)(a.rays_x * a.rays_y));
     pixel_of_item(a, b, tid, vm, x, y);
-    store_patch(a, vm, x, y, val, ok);
+    if (!spread)
+        store_patch(a, vm, x, y, val, ok);
+    else if (ok && ((x & (a.rays_x - 1u)) | (y & (a.rays_y - 1u))) == 0)
+        a.out[((size_t)vm * a.rows + (y >> a.sub_y)) * a.channels + (x >> a.sub_x)] = val;
 }
 
 constexpr int cell_maxreg(Mode m)

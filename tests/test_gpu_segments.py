@@ -179,3 +179,24 @@ def test_zero_voxels_outside_the_object_change_nothing(ctx, where, upsampling, s
         return
     want, _ = oracle.project_fp64(vol, (1.0, 1.2, 0.9), P, C, R, ray_sampling=sampling, upsampling=upsampling)
     assert want.max() > 0 and rel_err(got, want).max() <= 1e-4
+
+
+@pytest.mark.parametrize("rays", [(2, 1), (1, 4), (4, 4), (2, 4), (3, 2), (4, 8)])
+@pytest.mark.parametrize("kernel,upsampling", [(L.KERNEL_CELLS, 1), (L.KERNEL_PAIRS, 1), (L.KERNEL_AUTO, 2)])
+def test_sub_rays_on_lanes_of_their_own(ctx, rays, kernel, upsampling):
+    """1, 2 or 4 rays a side get a lane each, other counts run one after the other:
+    detectors that leave partial patches and tiles, and every launch shape the same bits."""
+    vol = _volume((18, 17, 23), 13)
+    C, R = 19, 11
+    P = _axis_views(C, R, 2.9, 0.17)
+    want, _ = oracle.project_fp64(vol, (1.0, 1.1, 1.2), P, C, R, rays=rays, upsampling=upsampling)
+    st = dict(rays_per_pixel=list(rays), kernel=kernel, volume_upsampling=upsampling)
+    v = ctx.volume(VoxelVolume(vol, (1.0, 1.1, 1.2)))
+    try:
+        got = ctx.project(v, P, C, R, Settings(**st))
+        assert rel_err(got, want).max() <= 1e-4
+        for block, views, lanes in ((128, 1, 4), (512, 4, 8), (128, 2, 8)):
+            other = ctx.project(v, P, C, R, Settings(block_rays=block, views_per_block=views, lanes_x=lanes, **st))
+            np.testing.assert_array_equal(other, got)
+    finally:
+        v.release()
