@@ -22,7 +22,7 @@ constexpr int kPad = 2;
 #define CTLCU_CELL_MAXREG 48  // cell and pair sample loops: 5 blocks of 256 threads per SM
 #endif
 #ifndef CTLCU_SEGMENT_MAXREG
-#define CTLCU_SEGMENT_MAXREG 64  // segment and up-sampled cell loops: 4 blocks of 256 threads per SM
+#define CTLCU_SEGMENT_MAXREG 64  // segment and up-sampled loops: 4 blocks of 256 threads per SM
 #endif
 #ifndef CTLCU_GATHER_MAXREG
 #define CTLCU_GATHER_MAXREG 80  // gather, nearest-voxel and texture loops: 3 blocks of 256 per SM
@@ -187,7 +187,7 @@ inline PairLayout pair_layout(const int n[3])
     return L;
 }
 
-enum class Mode : int { Trilinear = 0, Nearest = 1, Texture = 2, Cells = 3, Pairs = 4, Segments = 5, CellsUp = 6 };
+enum class Mode : int { Trilinear = 0, Nearest = 1, Texture = 2, Cells = 3, Pairs = 4, Segments = 5, CellsUp = 6, SegmentsUp = 7 };
 enum class Accum : int { F64 = 0, Kahan = 1, F32 = 2 };
 
 // Everything a projection launch needs, passed by value.
@@ -258,6 +258,13 @@ struct BatchReq {
 // The rule looks at the setting alone, so that a request takes the same loop in a
 // batch as on its own.
 constexpr float kSegmentMaxSampling = 0.6f;
+
+// Up-sampled f times, a stored voxel has two breaks (the ends of a ramp) along each
+// axis, 2 / f of the grid's, and a segment costs about 2.5 samples: segments up to a
+// ray_sampling of f / 6.  Segments / samples, ms, 101x97x89 -> 20 x 512 x 384:
+//   f = 2: 0.3 2.15 / 2.38, 0.4 2.07 / 1.82      f = 3: 0.5 2.12 / 2.15, 0.6 2.07 / 1.81
+//   f = 4: 0.6 2.15 / 2.38, 0.75 2.08 / 1.93     f = 7: 0.3 2.49 / 7.96, 1.0 2.16 / 2.49
+constexpr float kSegmentUpMaxSampling = 1.0f / 6.0f;
 
 // Launchers (raycast.cu / setup.cu / volume.cu).  All asynchronous on `s`.
 cudaError_t launch_batch_setup(const BatchSetup* reqs, uint32_t n_reqs, uint32_t total, ViewGeom* geom,

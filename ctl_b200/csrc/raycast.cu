@@ -169,7 +169,7 @@ __device__ __forceinline__ Ray setup_ray(const ProjectArgs& a, const ViewGeom& g
     return r;
 }
 
-// The same for the loops over derived arrays (Cells, Segments, CellsUp, Pairs).
+// The same for the loops over derived arrays (Cells, Segments, their up-sampled forms, Pairs).
 // Outside the box, padded by half a voxel, samples read zeros, so these loops run
 // over ceil(t0) .. floor(t1) of the slab intersection, which holds every sample that
 // the face tests above let in and that is not zero.  Lengths are in grid voxels from
@@ -203,7 +203,7 @@ __device__ __forceinline__ Ray setup_ray_cells(const ProjectArgs& a, const ViewG
     if (M != Mode::Pairs) {
         // clipped to the slabs of the cells that are not zero, a thousandth of a voxel
         // wider for the FP32 positions; cell i covers i - 1/2 .. i + 1/2 in v
-        const double f = M == Mode::CellsUp ? (double)a.up : 1.0;
+        const double f = M == Mode::CellsUp || M == Mode::SegmentsUp ? (double)a.up : 1.0;
         const double dir[5] = { d[0], d[1], d[2], d[0] + d[1], d[0] - d[1] };
         const double pos[5] = { s[0], s[1], s[2], s[0] + s[1], s[0] - s[1] };
         const double wide[5] = { 0.501, 0.501, 0.501, 1.002, 1.002 };
@@ -233,7 +233,7 @@ __device__ __forceinline__ Ray setup_ray_cells(const ProjectArgs& a, const ViewG
         for (int i = 0; i < 3; ++i) {
             r.base[i] = fma(i0, d[i], s[i]);
             r.step[i] = d[i];
-            if (M == Mode::CellsUp) {
+            if (M == Mode::CellsUp || M == Mode::SegmentsUp) {
                 // the same in stored voxels, a.up of the grid's to one
                 const double f = 1.0 / a.up;
                 r.base[i] *= f;
@@ -613,6 +613,117 @@ __device__ __forceinline__ void march_segments(const ProjectArgs& a, const Ray& 
     }
 }
 
+// One axis of a segment of the replicated grid.  Between the centres of two stored
+// voxels the grid is flat but for the ramp of one grid voxel about the face between
+// them, |f h| < 1/2 with h the offset from the cell's centre.  From h a ray along the
+// axis leaves its ramp, or its flat stretch (which runs on into the next cell), after
+// e steps; on the way the cell's own interpolant is taken at `at`, moving by `step`
+// per sample on the ramp and not at all off it.
+struct UpAxis {
+    float slope;       // -1 / step, as SegmentRay
+    float ramp, flat;  // steps from the cell's centre to the ramp's end, and to the next ramp
+    float step;        // f * step
+};
+
+__device__ __forceinline__ UpAxis up_axis(float d, float f)
+{
+    UpAxis u;
+    u.slope = exit_slope(d);
+    u.ramp = fabsf(u.slope) * (0.5f / f);
+    u.flat = fabsf(u.slope) * (1.0f - 0.5f / f);
+    u.step = f * d;
+    return u;
+}
+
+__device__ __forceinline__ float up_exit(const UpAxis& u, float h, float f, float& at, float& step)
+{
+    const float y = f * h;
+    const bool on = fabsf(y) < 0.5f;
+    // off the ramp: ahead of it where y and the step have opposite signs (slope and y the same)
+    const bool before = (__float_as_int(y) ^ __float_as_int(u.slope)) >= 0;
+    at = fminf(fmaxf(y, -0.5f), 0.5f);
+    step = on ? u.step : 0.0f;
+    return fmaf(h, u.slope, on ? u.ramp : (before ? -u.ramp : u.flat));
+}
+
+// One segment of the replicated grid, as cell_segment: the samples k .. of a ray up to
+// the nearest end of a ramp or a flat stretch, summed in closed form with the offsets
+// and steps of up_exit.  The cell is sample k's; where a flat stretch crosses into the
+// next cell, both cells hold the same values on it.
+__device__ __forceinline__ void cell_segment_up(const char* __restrict__ cells, float& k, float last,
+                                                const CellFrame& fr, float2 dxy, float dz, const UpAxis& ux,
+                                                const UpAxis& uy, const UpAxis& uz, float f, uint32_t sy, uint32_t sz,
+                                                uint32_t cmax, uint32_t offset, float& part)
+{
+    const float2 none2 = make_float2(-1.0f, -1.0f);
+    const float2 vxy = __ffma2_rn(make_float2(k, k), dxy, fr.bxy);
+    const float vz = fmaf(k, dz, fr.bz);
+    const float2 txy = __fadd2_rn(vxy, fr.mxy);
+    const float tz = __fadd_rn(vz, fr.mz);
+    const uint32_t idx = min(cell_linear(__float_as_uint(txy.x), __float_as_uint(txy.y), __float_as_uint(tz), sy, sz,
+                                         offset), cmax);
+    float c0, c1, c2, c3, c4, c5, c6, c7;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(c0), "=f"(c1), "=f"(c2), "=f"(c3), "=f"(c4), "=f"(c5), "=f"(c6), "=f"(c7)
+        : "l"(cells + (size_t)idx * kCellBytes));
+    const float2 hxy = __ffma2_rn(__ffma2_rn(fr.mxy, none2, txy), none2, vxy);
+    const float hz = __fsub_rn(vz, __fsub_rn(tz, fr.mz));
+    float ax, ay, az, sx, sy_, sz_;
+    const float ex = up_exit(ux, hxy.x, f, ax, sx), ey = up_exit(uy, hxy.y, f, ay, sy_), ez = up_exit(uz, hz, f, az, sz_);
+    const float e = fminf(fmaxf(min3(ex, ey, ez), 0.0f), last - k);
+    const float m = __fadd_rd(e, 8388608.0f) - 8388607.0f;
+    const float half = fmaf(m, 0.5f, -0.5f);
+    const float gx = fmaf(half, sx, ax), gy = fmaf(half, sy_, ay), gz = fmaf(half, sz_, az);
+    const float2 gx2 = make_float2(gx, gx);
+    const float2 ea = __ffma2_rn(gx2, make_float2(c2, c3), make_float2(c0, c1));
+    const float2 eb = __ffma2_rn(gx2, make_float2(c6, c7), make_float2(c4, c5));
+    const float2 g = __ffma2_rn(make_float2(gy, gy), eb, ea);
+    const float v = fmaf(gz, g.y, g.x);
+    // dx dy f_xy + dx dz f_xz + dy dz f_yz
+    const float q = fmaf(sx, fmaf(sz_, fmaf(gy, c7, c3), sy_ * fmaf(gz, c7, c6)), sy_ * sz_ * eb.y);
+    if (k <= last)
+        part = fmaf(m, fmaf(fmaf(m, m, -1.0f) * (1.0f / 12.0f), q, v), part);
+    k += m;
+}
+
+// march_segments for the replicated grid (positions in stored voxels).  101x97x89, f =
+// 3, 60 x 512 x 384 at the default step: 10.3 -> 6.6 ms against the sample loop.
+template <Accum ACC, int U>
+__device__ __forceinline__ void march_segments_up(const ProjectArgs& a, const Ray& r, Accumulator<ACC>& acc)
+{
+    const char* __restrict__ cells = static_cast<const char*>(a.cells);
+    CellFrame fr = cell_frame(r);
+    const float2 dxy = make_float2((float)r.step[0], (float)r.step[1]);
+    const float dz = (float)r.step[2], f = (float)a.up;
+    const float lx = (float)(r.step[0] - dxy.x), ly = (float)(r.step[1] - dxy.y), lz = (float)(r.step[2] - dz);
+    const UpAxis ux = up_axis(dxy.x, f), uy = up_axis(dxy.y, f), uz = up_axis(dz, f);
+    const uint32_t sy = a.csy, sz = a.csz, cmax = a.cmax, offset = a.coffset;
+    const bool hit = r.n > 0;
+    const int w1 = __reduce_max_sync(0xffffffffu, hit ? (r.first + r.n - 1) / kWindow : -1);
+    int w = __reduce_min_sync(0xffffffffu, hit ? r.first / kWindow : 0x7fffffff);
+    int at = r.first;
+    const int end = r.first + r.n;
+    for (; w <= w1; ++w) {
+        const int stop = min(end, (w + 1) * kWindow);
+        if (at < stop) {
+            const float last = (float)(stop - at - 1);
+            float k = 0.0f;
+            do {
+                float part = 0.0f;
+#pragma unroll
+                for (int j = 0; j < U; ++j)
+                    cell_segment_up(cells, k, last, fr, dxy, dz, ux, uy, uz, f, sy, sz, cmax, offset, part);
+                acc.add(part);
+            } while (k <= last);
+            advance_axis(fr.bxy.x, fr.mxy.x, dxy.x, lx, k);
+            advance_axis(fr.bxy.y, fr.mxy.y, dxy.y, ly, k);
+            advance_axis(fr.bz, fr.mz, dz, lz, k);
+            at = stop;
+        }
+        __syncwarp();
+    }
+}
+
 // Padded-array index of the voxel floor(p) of sample k, formed in FP64; beyond the
 // volume it is clamped to the array's zero border.
 __device__ __forceinline__ uint32_t nearest_index(const ProjectArgs& a, const Ray& r, int k)
@@ -910,6 +1021,8 @@ __device__ __forceinline__ void march_array(const ProjectArgs& a, const Ray& r, 
         march_pairs<ACC, U>(a, r, acc);
     else if (M == Mode::Segments)
         march_segments<ACC, U>(a, r, acc);
+    else if (M == Mode::SegmentsUp)
+        march_segments_up<ACC, U>(a, r, acc);
     else
         march_cells<ACC, U, M == Mode::CellsUp>(a, r, acc);
 }
@@ -927,7 +1040,7 @@ __device__ __forceinline__ void cells_item(const ProjectArgs& a, uint32_t b, uin
     const bool live = ok && g.valid;
     Accumulator<ACC> acc;
     // (up-sampled volumes with voxels that are no numbers, see gather_upsampled)
-    const bool by_voxel = M == Mode::CellsUp && __ldg(a.support + kSupportNonFinite) > 0;
+    const bool by_voxel = (M == Mode::CellsUp || M == Mode::SegmentsUp) && __ldg(a.support + kSupportNonFinite) > 0;
     auto ray = [&](double px, double py) {
         if (by_voxel) {
             gather_upsampled<ACC>(a, g, px, py, live, acc);
@@ -975,7 +1088,8 @@ __device__ __forceinline__ void cells_item(const ProjectArgs& a, uint32_t b, uin
 
 constexpr int cell_maxreg(Mode m)
 {
-    return m == Mode::Segments || m == Mode::CellsUp ? CTLCU_SEGMENT_MAXREG : CTLCU_CELL_MAXREG;
+    return m == Mode::Segments || m == Mode::SegmentsUp || m == Mode::CellsUp ? CTLCU_SEGMENT_MAXREG
+                                                                              : CTLCU_CELL_MAXREG;
 }
 
 // Cell, segment or pair loop over one block of the regular grid.
@@ -1106,7 +1220,10 @@ cudaError_t launch_typed(const ProjectArgs& a, int dtype, dim3 grid, cudaStream_
 }
 
 // Samples, or segments of about two samples, per partial sum of a loop.
-constexpr int loop_unroll(Mode m, int unroll) { return m == Mode::Segments ? unroll / 2 : unroll; }
+constexpr int loop_unroll(Mode m, int unroll)
+{
+    return m == Mode::Segments || m == Mode::SegmentsUp ? unroll / 2 : unroll;
+}
 
 template <Mode M, Accum ACC>
 cudaError_t launch_cells(const ProjectArgs& a, dim3 grid, cudaStream_t s)
@@ -1134,6 +1251,7 @@ cudaError_t launch_acc(const ProjectArgs& a, Mode mode, int dtype, dim3 grid, cu
     case Mode::Cells: return launch_cells<Mode::Cells, ACC>(a, grid, s);
     case Mode::Segments: return launch_cells<Mode::Segments, ACC>(a, grid, s);
     case Mode::CellsUp: return launch_cells<Mode::CellsUp, ACC>(a, grid, s);
+    case Mode::SegmentsUp: return launch_cells<Mode::SegmentsUp, ACC>(a, grid, s);
     case Mode::Pairs: return launch_cells<Mode::Pairs, ACC>(a, grid, s);
     }
     return cudaErrorInvalidValue;
