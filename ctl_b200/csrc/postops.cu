@@ -174,22 +174,26 @@ __device__ float noisy_count(double lam, Stream& s)
 // A pixel's draws do not depend on the lane or the round that makes them.  60 x 512^2
 // at 1e5 photons: 661 -> 356 us (a queue per block, whose barriers its warps
 // waited at: 367).
-constexpr uint32_t kNoiseTile = 1024;   // pixels per warp
+//
+// The tile is the largest, up to 1024 pixels, that still gives every SM 16 warps: few
+// pixels end up in partly filled rounds, while a small job keeps the GPU busy (2 x
+// 216 x 216: 30 us with tiles of 32, 63 with 1024, 32 before).
+constexpr uint32_t kNoiseTile = 1024;   // most pixels per warp
 constexpr uint32_t kNoiseWarps = 4;     // warps per block
 
 __global__ void __launch_bounds__(32 * kNoiseWarps)
     poisson_kernel(float* __restrict__ data, uint32_t n_views, uint32_t n_modules, uint32_t ppm,
-                   const float* __restrict__ i0, uint32_t k0, uint32_t k1)
+                   const float* __restrict__ i0, uint32_t k0, uint32_t k1, uint32_t tile)
 {
     __shared__ uint32_t stacks[kNoiseWarps][kNoiseTile];  // pixel of the tile | draw << 16
     uint32_t* stack = stacks[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
-    const uint32_t per_view = n_modules * ppm, tiles = (per_view - 1) / kNoiseTile + 1;
+    const uint32_t per_view = n_modules * ppm, tiles = (per_view - 1) / tile + 1;
     const uint64_t all = (uint64_t)tiles * n_views;
     for (uint64_t t = blockIdx.x * (uint64_t)kNoiseWarps + (threadIdx.x >> 5); t < all;
          t += gridDim.x * (uint64_t)kNoiseWarps) {
-        const uint32_t view = (uint32_t)(t / tiles), first = (uint32_t)(t - (uint64_t)view * tiles) * kNoiseTile;
-        const uint32_t n = min(kNoiseTile, per_view - first);
+        const uint32_t view = (uint32_t)(t / tiles), first = (uint32_t)(t - (uint64_t)view * tiles) * tile;
+        const uint32_t n = min(tile, per_view - first);
         float* p = data + (uint64_t)view * per_view + first;
         auto photons = [&](uint32_t j) { return i0[n_modules == 1 ? 0u : (first + j) / ppm]; };
         uint32_t held = 0;  // entries on the stack, the same in every lane
@@ -516,10 +520,14 @@ cudaError_t launch_poisson_noise(float* data, uint32_t n_views, uint32_t n_modul
     const uint64_t total = (uint64_t)n_views * n_modules * ppm;
     if (total == 0)
         return cudaSuccess;
-    const uint64_t tiles = ((uint64_t)n_modules * ppm - 1) / kNoiseTile + 1;
+    const uint64_t per_view = (uint64_t)n_modules * ppm;
+    uint32_t tile = kNoiseTile;
+    while (tile > 32u && total < 148ull * 16 * tile)
+        tile /= 2;
+    const uint64_t tiles = (per_view - 1) / tile + 1;
     const uint64_t blocks = std::min<uint64_t>((tiles * n_views + kNoiseWarps - 1) / kNoiseWarps, 148ull * 64);
     poisson_kernel<<<(unsigned)blocks, 32 * kNoiseWarps, 0, s>>>(data, n_views, n_modules, ppm, i0, (uint32_t)seed,
-                                                                 (uint32_t)(seed >> 32));
+                                                                 (uint32_t)(seed >> 32), tile);
     return cudaGetLastError();
 }
 
