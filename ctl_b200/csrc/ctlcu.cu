@@ -531,7 +531,8 @@ int volume_args(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, Project
 {
     const bool interp = s->interpolate != 0;
     const int f = interp ? (int)s->volume_upsampling : 1;  // no interpolation forces f = 1
-    mode = !interp ? Mode::Nearest : (s->interp_mode == CTLCU_INTERP_TEXTURE ? Mode::Texture : Mode::Trilinear);
+    const Mode nearest = s->ray_sampling <= kNearestSegmentMaxSampling ? Mode::Nearest : Mode::NearestSamples;
+    mode = !interp ? nearest : (s->interp_mode == CTLCU_INTERP_TEXTURE ? Mode::Texture : Mode::Trilinear);
     const ctlcu_volume_desc& d = v.desc;
     float voxel[3];
     a.tex = 0;

@@ -187,7 +187,7 @@ inline PairLayout pair_layout(const int n[3])
     return L;
 }
 
-enum class Mode : int { Trilinear = 0, Nearest = 1, Texture = 2, Cells = 3, Pairs = 4, Segments = 5, CellsUp = 6, SegmentsUp = 7 };
+enum class Mode : int { Trilinear = 0, Nearest = 1, Texture = 2, Cells = 3, Pairs = 4, Segments = 5, CellsUp = 6, SegmentsUp = 7, NearestSamples = 8 };
 enum class Accum : int { F64 = 0, Kahan = 1, F32 = 2 };
 
 // Everything a projection launch needs, passed by value.
@@ -265,6 +265,11 @@ constexpr float kSegmentMaxSampling = 0.6f;
 //   f = 2: 0.3 2.15 / 2.38, 0.4 2.07 / 1.82      f = 3: 0.5 2.12 / 2.15, 0.6 2.07 / 1.81
 //   f = 4: 0.6 2.15 / 2.38, 0.75 2.08 / 1.93     f = 7: 0.3 2.49 / 7.96, 1.0 2.16 / 2.49
 constexpr float kSegmentUpMaxSampling = 1.0f / 6.0f;
+
+// The nearest-voxel loop goes by segments up to this ray_sampling, above it sample by
+// sample in FP64.  Segments / samples, ms, 256^3 -> 15 x 512^2: 0.3 3.2 / 7.4, 0.75 2.78
+// / 3.10, 0.9 2.66 / 2.62, 1.0 2.56 / 2.38.
+constexpr float kNearestSegmentMaxSampling = 0.8f;
 
 // Launchers (raycast.cu / setup.cu / volume.cu).  All asynchronous on `s`.
 cudaError_t launch_batch_setup(const BatchSetup* reqs, uint32_t n_reqs, uint32_t total, ViewGeom* geom,

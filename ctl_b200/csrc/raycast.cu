@@ -120,7 +120,7 @@ __device__ __forceinline__ Ray setup_ray(const ProjectArgs& a, const ViewGeom& g
     const double s0 = g.src[0] / a.voxel[0], s1 = g.src[1] / a.voxel[1], s2 = g.src[2] / a.voxel[2];
     const double k0 = a.corner[0] / a.voxel[0], k1 = a.corner[1] / a.voxel[1],
                  k2 = a.corner[2] / a.voxel[2];
-    const double pad = (M == Mode::Nearest) ? 0.0 : 0.5;
+    const double pad = (M == Mode::Nearest || M == Mode::NearestSamples) ? 0.0 : 0.5;
     const double c10 = k0 - pad, c11 = k1 - pad, c12 = k2 - pad;
     const double c20 = k0 + a.grid[0] + pad, c21 = k1 + a.grid[1] + pad, c22 = k2 + a.grid[2] + pad;
     const double l10 = (c10 - s0) / d0, l11 = (c11 - s1) / d1, l12 = (c12 - s2) / d2;
@@ -156,7 +156,7 @@ __device__ __forceinline__ Ray setup_ray(const ProjectArgs& a, const ViewGeom& g
     double shift;
     if (M == Mode::Trilinear)
         shift = (a.up == 1) ? (kPad - 0.5) : -0.5;  // taps at floor(p - 0.5) (+ pad)
-    else if (M == Mode::Nearest)
+    else if (M == Mode::Nearest || M == Mode::NearestSamples)
         shift = kPad;                                // voxel floor(p) (+ pad)
     else
         shift = 0.0;                                 // texture: hardware subtracts 0.5
@@ -833,6 +833,16 @@ __device__ __forceinline__ void march_nearest(const ProjectArgs& a, const Ray& r
         acc.add(load_voxel(vol + nearest_index(a, r, r.n - 1)));
 }
 
+// The same, every sample on its own: the faster form where a voxel holds hardly more
+// than one (kNearestSegmentMaxSampling).
+template <typename T, Accum ACC>
+__device__ __forceinline__ void march_nearest_samples(const ProjectArgs& a, const Ray& r, Accumulator<ACC>& acc)
+{
+    const T* __restrict__ vol = static_cast<const T*>(a.vol);
+    for (int k = 0; k < r.n; ++k)
+        acc.add(load_voxel(vol + nearest_index(a, r, k)));
+}
+
 // x-pair entries of the current cell: rows (y, z), (y+1, z), (y, z+1), (y+1, z+1).
 struct PairCache {
     uint32_t idx = 0xffffffffu;
@@ -923,6 +933,8 @@ __device__ __forceinline__ void march_texture(const ProjectArgs& a, const Ray& r
 // Pixel (with sub-rays spread over lanes, sub-ray of the finer grid of channels <<
 // sub_x by rows << sub_y) of thread `tid` of work item (block) `b` of a.block threads, for the
 // launch shape in `a` (every factor of the mapping is a power of two).
+// ROWS: consecutive lanes run down the rows of a channel, else along the channels.
+template <bool ROWS>
 __device__ __forceinline__ bool pixel_of_item(const ProjectArgs& a, uint32_t b, uint32_t tid, uint32_t& vm,
                                               uint32_t& x, uint32_t& y)
 {
@@ -946,18 +958,21 @@ __device__ __forceinline__ bool pixel_of_item(const ProjectArgs& a, uint32_t b, 
     const uint32_t view = (vg << a.vpb_shift) + slot;
     vm = view * a.n_modules + m;
     const uint32_t ty = t / a.tiles_x, tx = t - ty * a.tiles_x;
-    // consecutive lanes run down the rows of a channel: their rays share x and y and
-    // differ in z, which the cell layout serves without conflicts (CellLayout)
+    // rays down the rows of a channel share x and y and differ in z, which the cell
+    // layout serves without conflicts (CellLayout); along the channels they share lines
+    // of the voxel array, x fastest
     const uint32_t ly_shift = 5u - a.lx_shift;
-    x = (tx << a.tx_shift) + ((w & ((1u << a.wx_shift) - 1u)) << a.lx_shift) + (lane >> ly_shift);
-    y = (ty << a.ty_shift) + ((w >> a.wx_shift) << ly_shift) + (lane & ((1u << ly_shift) - 1u));
+    const uint32_t lx = ROWS ? lane >> ly_shift : lane & ((1u << a.lx_shift) - 1u);
+    const uint32_t ly = ROWS ? lane & ((1u << ly_shift) - 1u) : lane >> a.lx_shift;
+    x = (tx << a.tx_shift) + ((w & ((1u << a.wx_shift) - 1u)) << a.lx_shift) + lx;
+    y = (ty << a.ty_shift) + ((w >> a.wx_shift) << ly_shift) + ly;
     return view < a.n_views && x < a.span_x && y < a.span_y;
 }
 
 __device__ __forceinline__ bool pixel_of_thread(const ProjectArgs& a, uint32_t tid, uint32_t& vm, uint32_t& x,
                                                 uint32_t& y)
 {
-    return pixel_of_item(a, blockIdx.x, tid, vm, x, y);
+    return pixel_of_item<false>(a, blockIdx.x, tid, vm, x, y);
 }
 
 __device__ __forceinline__ bool pixel_of(const ProjectArgs& a, uint32_t& vm, uint32_t& x, uint32_t& y)
@@ -967,16 +982,17 @@ __device__ __forceinline__ bool pixel_of(const ProjectArgs& a, uint32_t& vm, uin
 
 // Writes the warp's pixel values (called by all 32 lanes): each lane holds
 // `val` for pixel (vm, x, y), or ok = false for no pixel.  The lanes of four
-// consecutive channels of one detector row lie one patch height apart (a warp
-// patch is 4 or 8 channels wide); where all four pixels exist and their row
+// consecutive channels of one detector row follow each other, or lie one patch height
+// apart (ROWS; a warp patch is 4 or 8 channels wide); where all four pixels exist and their row
 // segment starts on a 16-byte boundary, the first of them gathers the other three
 // values and writes the segment as one 16-byte store; otherwise each lane stores
 // its own value.
+template <bool ROWS>
 __device__ __forceinline__ void store_patch(const ProjectArgs& a, uint32_t vm, uint32_t x, uint32_t y, float val,
                                             bool ok)
 {
     const uint32_t full = 0xffffffffu, lane = threadIdx.x & 31u;
-    const uint32_t ls = 5u - a.lx_shift;  // log2 of the patch height
+    const uint32_t ls = ROWS ? 5u - a.lx_shift : 0u;  // log2 of the lanes from a channel to the next
     const uint32_t lead = lane & ~(3u << ls);
     const float v1 = __shfl_down_sync(full, val, 1u << ls);
     const float v2 = __shfl_down_sync(full, val, 2u << ls);
@@ -1035,7 +1051,7 @@ template <Mode M, Accum ACC, int U>
 __device__ __forceinline__ void cells_item(const ProjectArgs& a, uint32_t b, uint32_t tid)
 {
     uint32_t vm, x, y;
-    const bool ok = pixel_of_item(a, b, tid, vm, x, y);
+    const bool ok = pixel_of_item<true>(a, b, tid, vm, x, y);
     const ViewGeom& g = a.geom[ok ? vm : 0u];
     const bool live = ok && g.valid;
     Accumulator<ACC> acc;
@@ -1058,8 +1074,8 @@ __device__ __forceinline__ void cells_item(const ProjectArgs& a, uint32_t b, uin
         ray((double)x, (double)y);
         const float val = static_cast<float>(a.increment * acc.value());
         // the pixel again for the store, rather than holding it through the loop
-        pixel_of_item(a, b, tid, vm, x, y);
-        store_patch(a, vm, x, y, val, ok);
+        pixel_of_item<true>(a, b, tid, vm, x, y);
+        store_patch<true>(a, vm, x, y, val, ok);
         return;
     }
     const bool spread = (a.sub_x | a.sub_y) != 0;  // a lane per sub-ray
@@ -1079,9 +1095,9 @@ __device__ __forceinline__ void cells_item(const ProjectArgs& a, uint32_t b, uin
             sum += __shfl_xor_sync(0xffffffffu, sum, o << ls);
     }
     const float val = static_cast<float>(a.increment * sum / (double)(a.rays_x * a.rays_y));
-    pixel_of_item(a, b, tid, vm, x, y);
+    pixel_of_item<true>(a, b, tid, vm, x, y);
     if (!spread)
-        store_patch(a, vm, x, y, val, ok);
+        store_patch<true>(a, vm, x, y, val, ok);
     else if (ok && ((x & (a.rays_x - 1u)) | (y & (a.rays_y - 1u))) == 0)
         a.out[((size_t)vm * a.rows + (y >> a.sub_y)) * a.channels + (x >> a.sub_x)] = val;
 }
@@ -1150,7 +1166,7 @@ __global__ void __maxnreg__(cell_maxreg(M))
 template <typename T, Mode M, Accum ACC, bool UP>
 __global__ void __maxnreg__(CTLCU_GATHER_MAXREG) project_kernel(const __grid_constant__ ProjectArgs a)
 {
-    static_assert(M == Mode::Trilinear || M == Mode::Nearest || M == Mode::Texture, "cells_kernel runs these");
+    static_assert(M == Mode::Trilinear || M == Mode::Nearest || M == Mode::NearestSamples || M == Mode::Texture, "cells_kernel runs these");
     uint32_t vm, x, y;
     const bool ok = pixel_of(a, vm, x, y);
     const ViewGeom& g = a.geom[ok ? vm : 0u];
@@ -1168,11 +1184,13 @@ __global__ void __maxnreg__(CTLCU_GATHER_MAXREG) project_kernel(const __grid_con
                 march_trilinear<T, ACC, UP>(a, r, acc);
             else if (M == Mode::Nearest)
                 march_nearest<T, ACC>(a, r, acc);
+            else if (M == Mode::NearestSamples)
+                march_nearest_samples<T, ACC>(a, r, acc);
             else
                 march_texture<ACC>(a, r, acc);
         }
     const float val = static_cast<float>(a.increment * acc.value() / (double)(a.rays_x * a.rays_y));
-    store_patch(a, vm, x, y, val, ok);
+    store_patch<false>(a, vm, x, y, val, ok);
 }
 
 template <Mode M>
@@ -1245,6 +1263,7 @@ cudaError_t launch_acc(const ProjectArgs& a, Mode mode, int dtype, dim3 grid, cu
         return a.up != 1 ? launch_typed<Mode::Trilinear, ACC, true>(a, dtype, grid, s)
                          : launch_typed<Mode::Trilinear, ACC, false>(a, dtype, grid, s);
     case Mode::Nearest: return launch_typed<Mode::Nearest, ACC, false>(a, dtype, grid, s);
+    case Mode::NearestSamples: return launch_typed<Mode::NearestSamples, ACC, false>(a, dtype, grid, s);
     case Mode::Texture:
         project_kernel<float, Mode::Texture, ACC, false><<<grid, a.block, 0, s>>>(a);
         return cudaGetLastError();
@@ -1353,7 +1372,7 @@ cudaError_t launch_count(const ProjectArgs& a, Mode mode, cudaStream_t s)
     if (blocks > 0x7fffffffull || !block_ok(a))
         return cudaErrorInvalidConfiguration;
     const dim3 grid((unsigned)blocks);
-    if (mode == Mode::Nearest)
+    if (mode == Mode::Nearest || mode == Mode::NearestSamples)
         count_kernel<Mode::Nearest><<<grid, a.block, 0, s>>>(a);
     else
         count_kernel<Mode::Trilinear><<<grid, a.block, 0, s>>>(a);
