@@ -56,10 +56,10 @@ N_VIEWS = 360
 METRIC = "projections/s at 256\u00b3\u2192512\u00b2 (plain FP32 vs batched BF16); p50/p99 DRR latency"
 WORKLOAD = "256^3 f32 ellipsoid phantom -> 360 x 512^2 short-scan (200 deg + fan), raySampling 0.3, trilinear"
 # DRAM bytes (read + write) of one 360-view launch of the cell loop on this
-# workload, from one ncu capture (profiles/cells_kernel_256cubed_to_512sq_dram.md),
+# workload, from one ncu capture (profiles/segments_kernel_201x173x155.md),
 # with the launch shape it was captured at (views per block, lanes_x, rays per block, unroll)
 # and its accumulator
-CELLS_TRAFFIC_BYTES = 7.883831808e9 + 0.424111872e9
+CELLS_TRAFFIC_BYTES = 6.114473472e9 + 0.380621056e9
 CELLS_TRAFFIC_SHAPE = (2, 4, 256, 4)
 CELLS_TRAFFIC_ACCUM = "kahan"
 
@@ -383,6 +383,9 @@ def run_ours(args):
                          "frac": achieved / l1_peak, "traffic": traffic,
                          "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one full launch"
                                            if traffic else "not captured for this variant",
+                         # the scheme's eight taps per sample; the segment loop reads one 32-byte cell
+                         # for all samples a ray has in it, so this fraction can exceed 1
+                         "algorithmic": "8 taps x stored bytes per sample of the reference scheme + output",
                          "peak_source": f"{sms} SMs x 128 B/clk x {mhz:.0f} MHz sampled SM clock",
                          "algorithmic_bytes_per_launch": alg_bytes,
                          # the DRAM side: the captured traffic over this run's launch time, against
