@@ -134,6 +134,7 @@ __device__ __forceinline__ Ray setup_ray(const ProjectArgs& a, const ViewGeom& g
     check_face(s0 + l21 * d0, s2 + l21 * d2, c10 - e, c12 - e, c20 + e, c22 + e, l21, tmin, tmax);
     check_face(s0 + l22 * d0, s1 + l22 * d1, c10 - e, c11 - e, c20 + e, c21 + e, l22, tmin, tmax);
     r.n = 0;
+    r.first = 0;
     if (tmin == DBL_MAX) {
         r.base[0] = r.base[1] = r.base[2] = 0.0;
         r.step[0] = r.step[1] = r.step[2] = 0.0;
@@ -780,12 +781,14 @@ __device__ __forceinline__ void march_nearest(const ProjectArgs& a, const Ray& r
     const float lo = 0.5f - del, hi = 0.5f + del;
     const uint32_t sy = (uint32_t)a.sy, sz = (uint32_t)a.sz, offset = 0u - kMagicBits * (1u + sy + sz);
     const float2 none2 = make_float2(-1.0f, -1.0f);
-    const bool hit = at < end;
+    // the number of samples alone says whether a ray takes part: one that misses has no
+    // place along the ray to compare
+    const bool hit = r.n > 2;
     const int w1 = __reduce_max_sync(0xffffffffu, hit ? (end - 1) / kWindow : -1);
     int w = __reduce_min_sync(0xffffffffu, hit ? at / kWindow : 0x7fffffff);
     for (; w <= w1; ++w) {
         const int stop = min(end, (w + 1) * kWindow);
-        if (at < stop) {
+        if (hit && at < stop) {
             const float last = (float)(stop - at - 1);
             float k = 0.0f;
             do {
