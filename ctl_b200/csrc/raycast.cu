@@ -778,7 +778,16 @@ __device__ __forceinline__ void march_nearest(const ProjectArgs& a, const Ray& r
     int at = r.first + 1;
     const float reach = (float)kWindow * fmaxf(fmaxf(fabsf(dxy.x), fabsf(dxy.y)), fabsf(dz)) + 1.0f;
     const float del = 1.5e-7f * reach + 2.5e-7f * ((float)(r.n / kWindow) + 4.0f);
-    const float lo = 0.5f - del, hi = 0.5f + del;
+    // A source so far away that FP64 cannot hold a position to a voxel (1e16 voxels; any
+    // finite matrix is served) puts samples anywhere.  FP32 decides only where the samples
+    // taken here stay within a voxel of the volume, a voxel inside the padded array; for
+    // other rays `lo` leaves every sample to nearest_run, which holds its indexes in the array.
+    bool inside = true;
+    for (int i = 0; i < 3; ++i) {
+        const double p0 = r.base[i] + r.step[i], p1 = fma((double)(r.n - 2), r.step[i], r.base[i]);
+        inside = inside && fmin(p0, p1) >= kPad - 1.0 && fmax(p0, p1) < a.ext[i] - 1.0;
+    }
+    const float lo = inside ? 0.5f - del : -1.0f, hi = 0.5f + del;
     const uint32_t sy = (uint32_t)a.sy, sz = (uint32_t)a.sz, offset = 0u - kMagicBits * (1u + sy + sz);
     const float2 none2 = make_float2(-1.0f, -1.0f);
     // the number of samples alone says whether a ray takes part: one that misses has no

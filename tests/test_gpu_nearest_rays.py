@@ -1,5 +1,6 @@
 """The nearest-voxel loop on rays that its fast road must not take on trust: warps
-in which some or all rays miss the volume."""
+in which some or all rays miss the volume, and sources so far away that FP64 no
+longer places a sample."""
 import numpy as np
 import pytest
 
@@ -53,5 +54,57 @@ def test_rays_that_miss_add_nothing(ctx, storage, sampling):
             got = ctx.project(v, P, C, R, Settings(ray_sampling=sampling, accum=accum, interpolate=False))
             np.testing.assert_array_equal(got[want == 0], 0.0)
             assert rel_err(got, want).max() <= 1e-4
+    finally:
+        v.release()
+
+
+def _inner_positions(P, channels, rows, n, voxel, sampling):
+    """Voxel positions of the second and the last but one sample of each ray that the
+    face tests let in, in FP64 as the ray setup forms them (one voxel size)."""
+    inc = sampling * voxel
+    qr, src = (x.ravel() for x in oracle.view_setup(P[None, None]))
+    up = np.array([[qr[9], qr[10], qr[11]], [0.0, qr[12], qr[13]], [0.0, 0.0, qr[14]]])
+    A, out = np.linalg.solve(up, qr[:9].reshape(3, 3).T), []
+    s, k, n = src / voxel, -0.5 * np.asarray(n, float), np.asarray(n, float)
+    for y in range(rows):
+        for x in range(channels):
+            d = A @ np.array([x, y, 1.0])
+            d *= inc / voxel / np.sqrt(d @ d)
+            with np.errstate(all="ignore"):
+                hits = [l for l, face in [((c[a] - s[a]) / d[a], a) for c in (k, k + n) for a in range(3)]
+                        if all(k[i] - 0.01 <= s[i] + l * d[i] <= k[i] + n[i] + 0.01 for i in range(3) if i != face)]
+            i0, i1 = (np.floor(max(min(hits), 0.0)), np.floor(max(hits)) + 1) if hits else (0, 0)
+            if i1 - i0 < 2:
+                continue  # two samples, both taken on their own
+            base = (s - k) + i0 * d
+            out += [base + d, base + (i1 - i0 - 1) * d]
+    return np.array(out)
+
+
+@pytest.mark.parametrize("far", [1e8, 1e16, 1e17, 1e18, 1e25])
+@pytest.mark.parametrize("storage", [L.F32, L.F16])
+def test_sources_beyond_what_fp64_places(ctx, far, storage):
+    """Any finite matrix is served.  From 1e16 voxels on the positions are off by more
+    than the array's border, samples may land anywhere, and those outside the volume read
+    zeros.  The volume is 1 everywhere: a pixel's value is its samples in the volume
+    times the step, so no sum exceeds the sample count, and nothing is not a number."""
+    n, voxel, C, R = (20, 18, 19), 1.0, 24, 17
+    vol = np.ones(n[::-1], np.float32)
+    u = np.array([0.83, 0.41, 0.37]) / np.linalg.norm([0.83, 0.41, 0.37])
+    P = _view(far * u, (0, 0, 0), C, R, 1.0, sdd=far)[None, None]
+    inner = _inner_positions(P[0, 0], C, R, n, voxel, 0.3)
+    beyond = max((-inner).max(), (inner - np.array(n)).max()) if len(inner) else 0.0
+    assert beyond < 0.02 if far < 1e10 else far != 1e17 or beyond > 4  # 1e17 reaches past the border
+    v = ctx.volume(VoxelVolume(vol, (voxel,) * 3), storage)
+    try:
+        st = dict(ray_sampling=0.3, interpolate=False)
+        samples = ctx.count_samples(v, P, C, R, Settings(**st))
+        for accum in (L.ACCUM_KAHAN, L.ACCUM_FP64):
+            got = ctx.project(v, P, C, R, Settings(accum=accum, **st))
+            assert np.isfinite(got).all() and got.min() >= 0.0
+            assert got.sum() <= 0.3 * samples * (1 + 1e-5)
+            if far < 1e10:
+                want, _ = oracle.project_fp64(vol, (voxel,) * 3, P, C, R, **st)
+                assert rel_err(got, want).max() <= 0.02  # a sample on a face may count to either side
     finally:
         v.release()
