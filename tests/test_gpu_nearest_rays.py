@@ -1,6 +1,6 @@
 """The nearest-voxel loop on rays that its fast road must not take on trust: warps
-in which some or all rays miss the volume, and sources so far away that FP64 no
-longer places a sample."""
+in which some or all rays miss the volume, sources so far away that FP64 no longer
+places a sample, and sums that FP32 cannot hold."""
 import numpy as np
 import pytest
 
@@ -106,5 +106,42 @@ def test_sources_beyond_what_fp64_places(ctx, far, storage):
             if far < 1e10:
                 want, _ = oracle.project_fp64(vol, (voxel,) * 3, P, C, R, **st)
                 assert rel_err(got, want).max() <= 0.02  # a sample on a face may count to either side
+    finally:
+        v.release()
+
+
+@pytest.mark.parametrize("storage", [L.F32, L.F16])
+@pytest.mark.parametrize("sampling", [0.02, 0.3, 0.8, 0.81])
+def test_fp64_accumulator_sums_the_samples_without_fp32_rounding(ctx, storage, sampling):
+    """Voxels of both signs, full mantissas, whose sums along a ray nearly cancel.  The
+    oracle and an FP64 accumulator differ by the order of at most a few hundred FP64
+    additions, below 1e-12 of the sum of magnitudes, and each rounds its result to FP32
+    once: one unit in the last place of FP32 (1.2e-7).  A product or a sum of two voxels
+    rounded to FP32 shows as 1e-8 of the sum of magnitudes, which exceeds the result by
+    a factor of several here.  A sample in a neighbouring voxel shows as a hundredth
+    of it.  Pixels with a sample on a face, either of whose voxels is right, are those
+    whose oracle value jumps under a shift of 1e-9 pixel."""
+    rng = np.random.default_rng(17)
+    vol = rng.uniform(0.5, 1.0, (24, 26, 28)) * np.where(np.indices((24, 26, 28)).sum(0) % 2, 1.0, -1.0)
+    vol = vol.astype(np.float16 if storage == L.F16 else np.float32).astype(np.float32)
+    voxel, C, R = (1.0, 1.1, 1.2), 45, 31
+    P = np.stack([_view((900, 31, 7), (0, 0, 0), C, R, 0.9), _view((7, 31, 900), (0, 0, 0), C, R, 0.9),
+                  _view((500, 600, 400), (0, 0, 0), C, R, 0.9)])[:, None]
+    st = dict(ray_sampling=sampling, interpolate=False)
+    want, _ = oracle.project_fp64(vol, voxel, P, C, R, **st)
+    total, _ = oracle.project_fp64(np.abs(vol), voxel, P, C, R, **st)
+    assert np.median(np.abs(want[total > 0]) / total[total > 0]) < 0.2
+    ties = np.zeros(want.shape, bool)
+    for shift in ((1e-9, 1e-9), (-1e-9, -1e-9), (1e-9, -1e-9), (-1e-9, 1e-9)):
+        moved = np.eye(3)
+        moved[:2, 2] = shift
+        near, _ = oracle.project_fp64(vol, voxel, moved @ P, C, R, **st)
+        ties |= np.abs(near - want) > 1e-6 * total
+    assert ties.mean() < 0.01
+    v = ctx.volume(VoxelVolume(vol, voxel), storage)
+    try:
+        got = ctx.project(v, P, C, R, Settings(accum=L.ACCUM_FP64, **st))
+        err = np.abs(got.astype(float) - want)
+        assert (err <= 1.2e-7 * np.abs(want) + 1e-12 * total)[~ties].all()
     finally:
         v.release()
