@@ -200,3 +200,34 @@ def test_sub_rays_on_lanes_of_their_own(ctx, rays, kernel, upsampling):
             np.testing.assert_array_equal(other, got)
     finally:
         v.release()
+
+
+@pytest.mark.parametrize("upsampling,step,bits", [(1, 3 / 128, 15), (2, 3 / 128, 15), (4, 3 / 128, 15),
+                                                  (2, 3 / 16, 21), (4, 3 / 16, 21)])
+def test_fp64_accumulator_adds_no_rounding(ctx, upsampling, step, bits):
+    """Rays along the middle rows of 3 x 3 equal rows of voxels, at steps of 3/128 or 3/16
+    voxel, through whole numbers of `bits` bits: sample positions, coefficients and
+    interpolants all fit FP32's 24 bits, so the value of every sample, and of every cell
+    at the midpoint of its samples, is exact (at a multiple of 1/256 of a voxel and of
+    1/8).  Only sums can round: four cells of 42 samples, or eight samples, need more than
+    24 bits, an FP64 accumulator holds them all, and the result equals the oracle's,
+    rounded to FP32 once."""
+    n = (18, 36, 36)
+    vol = np.random.default_rng(23).integers(0, 1 << bits, (12, 12, 18)).astype(np.float32)
+    vol = vol.repeat(3, 0).repeat(3, 1)
+    K = G.intrinsic(1024.0, 1.0, 1.0, 0.0, 0.0)
+    P = []
+    for z in range(1, n[2], 3):
+        for y in range(1, n[1], 3):
+            src = np.array([512.0, y + 0.5 - n[1] / 2, z + 0.5 - n[2] / 2])
+            P.append(G.compose(K, G.camera_rotation(np.array([-1.0, 0.0, 0.0]), np.array([0.0, 0.0, 1.0])), src))
+    P = np.stack(P)[:, None]
+    st = dict(ray_sampling=step * upsampling)
+    want, samples = oracle.project_fp64(vol, (1.0, 1.0, 1.0), P, 1, 1, upsampling=upsampling, **st)
+    assert samples > len(P) * n[0] / step and (want > 0).all()
+    v = ctx.volume(VoxelVolume(vol, (1.0, 1.0, 1.0)))
+    try:
+        got = ctx.project(v, P, 1, 1, Settings(volume_upsampling=upsampling, accum=L.ACCUM_FP64, unroll=8, **st))
+        np.testing.assert_array_equal(got, want)
+    finally:
+        v.release()
