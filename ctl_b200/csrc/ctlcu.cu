@@ -712,7 +712,8 @@ int project_device(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s_in, c
     ProjectArgs a = {};
     Mode mode;
     int dtype;
-    int r = volume_args(ctx, v, s, a, mode, dtype);
+    // a stream that is ordered already is so after the arrays there are: it builds none
+    int r = volume_args(ctx, v, s, a, mode, dtype, !st_ordered);
     if (r)
         return r;
     if (!st_ordered) {
@@ -812,7 +813,8 @@ int project_any(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, const d
         if (!ctx->aux_stream)
             CU_TRY(ctx, cudaStreamCreateWithFlags(&ctx->aux_stream, cudaStreamNonBlocking));
         // the second stream starts after the pmats upload, the volume staging and
-        // the derived arrays, which are built here rather than by the first chunk
+        // the derived arrays, which are built here and by no chunk, so that one loop
+        // serves them all
         {
             const ctlcu_settings eff = resolve_kernel(ctx, v, s, C, R, M);
             ProjectArgs a = {};

@@ -1,0 +1,35 @@
+"""What the host side does around its launches, on a simulated CUDA runtime
+(tests/hostsim): the order of streams, and arrays built and freed."""
+import pytest
+
+import hostsim
+from ctl_b200 import _lib as L
+
+
+@pytest.fixture(scope="module")
+def library(tmp_path_factory):
+    return hostsim.build(str(tmp_path_factory.mktemp("hostsim")))
+
+
+@pytest.fixture
+def sim(library):
+    s = hostsim.Sim(library)
+    yield s
+    s.close()
+
+
+@pytest.mark.parametrize("answers", [[1000, 1 << 30], [1000] * 3 + [1 << 30], [1 << 30, 1000], [1 << 30]])
+@pytest.mark.parametrize("views", [5, 40, 100])
+def test_a_host_result_comes_from_one_loop_ordered_after_its_array(sim, answers, views):
+    """Up-sampled projections into host memory, in chunks on two streams, while the free
+    memory changes between any two looks at it: one loop serves the whole call, and no
+    chunk reads cells that its stream is not ordered after."""
+    v, _ = sim.volume()
+    sim.clear()
+    sim.free_answers(answers + [answers[-1]] * 20)
+    assert sim.project(v, sim.settings(volume_upsampling=2), views=views, host=True) == L.OK
+    launches = sim.projections()
+    assert sum(p[1] for p in launches) == views
+    assert {p[0] for p in launches} == {hostsim.GATHER if answers[0] == 1000 else hostsim.SEGMENTS_UP}
+    assert all(p[4] in ("-", "ok") for p in launches)
+    assert len({p[2] for p in launches}) == (2 if views >= 8 else 1)
