@@ -323,6 +323,33 @@ int make_volume(ctlcu_ctx* ctx, const ctlcu_volume_desc* d, const float* data, b
     return CTLCU_OK;
 }
 
+// Frees the volume's coefficient cells (pair entries), if it has any.
+void drop_cells(ctlcu_ctx* ctx, VolumeEntry& v)
+{
+    if (!v.cells)
+        return;
+    if (v.pooled)
+        cudaFreeAsync(v.cells, ctx->stream);
+    else
+        cudaFree(v.cells);
+    ctx->used -= std::min<uint64_t>(ctx->used, v.cell_bytes);
+    v.cells = nullptr;
+    v.cell_bytes = 0;
+}
+
+void drop_pairs(ctlcu_ctx* ctx, VolumeEntry& v)
+{
+    if (!v.pairs)
+        return;
+    if (v.pooled)
+        cudaFreeAsync(v.pairs, ctx->stream);
+    else
+        cudaFree(v.pairs);
+    ctx->used -= std::min<uint64_t>(ctx->used, v.pair_bytes);
+    v.pairs = nullptr;
+    v.pair_bytes = 0;
+}
+
 void free_volume(ctlcu_ctx* ctx, VolumeEntry& v)
 {
     for (auto& t : v.tex) {
@@ -336,24 +363,8 @@ void free_volume(ctlcu_ctx* ctx, VolumeEntry& v)
     if (v.mean)
         cudaFreeAsync(v.mean, ctx->stream);
     v.mean = nullptr;
-    if (v.cells) {
-        if (v.pooled)
-            cudaFreeAsync(v.cells, ctx->stream);
-        else
-            cudaFree(v.cells);
-        ctx->used -= std::min<uint64_t>(ctx->used, v.cell_bytes);
-    }
-    v.cells = nullptr;
-    v.cell_bytes = 0;
-    if (v.pairs) {
-        if (v.pooled)
-            cudaFreeAsync(v.pairs, ctx->stream);
-        else
-            cudaFree(v.pairs);
-        ctx->used -= std::min<uint64_t>(ctx->used, v.pair_bytes);
-    }
-    v.pairs = nullptr;
-    v.pair_bytes = 0;
+    drop_cells(ctx, v);
+    drop_pairs(ctx, v);
     if (v.data) {
         if (v.pooled)
             cudaFreeAsync(v.data, ctx->stream);
@@ -402,7 +413,11 @@ int ensure_cells(ctlcu_ctx* ctx, VolumeEntry& v)
         CU_TRY(ctx, cudaMalloc(&v.cells, bytes));
     v.cell_bytes = bytes;
     ctx->used += bytes;
-    CU_TRY(ctx, launch_build_cells(v.data, n, v.desc.dtype, L, v.cells, ctx->stream));
+    const cudaError_t e = launch_build_cells(v.data, n, v.desc.dtype, L, v.cells, ctx->stream);
+    if (e != cudaSuccess) {
+        drop_cells(ctx, v);
+        return fail(ctx, CTLCU_ERR_CUDA, "building the cell array failed: %s", cudaGetErrorString(e));
+    }
     ++ctx->launches;
     return CTLCU_OK;
 }
@@ -425,7 +440,11 @@ int ensure_pairs(ctlcu_ctx* ctx, VolumeEntry& v)
         CU_TRY(ctx, cudaMalloc(&v.pairs, bytes));
     v.pair_bytes = bytes;
     ctx->used += bytes;
-    CU_TRY(ctx, launch_build_pairs(v.data, n, v.desc.dtype, L, v.pairs, ctx->stream));
+    const cudaError_t e = launch_build_pairs(v.data, n, v.desc.dtype, L, v.pairs, ctx->stream);
+    if (e != cudaSuccess) {
+        drop_pairs(ctx, v);
+        return fail(ctx, CTLCU_ERR_CUDA, "building the pair array failed: %s", cudaGetErrorString(e));
+    }
     ++ctx->launches;
     return CTLCU_OK;
 }
@@ -2092,18 +2111,10 @@ int ctlcu_autotune(ctlcu_ctx* ctx, uint64_t volume, const ctlcu_settings* settin
     ctx->tuned[std::make_tuple(volume, channels, rows, n_modules)] = ctlcu_ctx::Tuned{ cand[best], shape_of(&bs) };
     // keep only the array the chosen loop reads
     cudaStreamSynchronize(ctx->stream);
-    if (cand[best] != CTLCU_KERNEL_CELLS && v->cells) {
-        cudaFree(v->cells);
-        ctx->used -= std::min<uint64_t>(ctx->used, v->cell_bytes);
-        v->cells = nullptr;
-        v->cell_bytes = 0;
-    }
-    if (cand[best] != CTLCU_KERNEL_PAIRS && v->pairs) {
-        cudaFree(v->pairs);
-        ctx->used -= std::min<uint64_t>(ctx->used, v->pair_bytes);
-        v->pairs = nullptr;
-        v->pair_bytes = 0;
-    }
+    if (cand[best] != CTLCU_KERNEL_CELLS)
+        drop_cells(ctx, *v);
+    if (cand[best] != CTLCU_KERNEL_PAIRS)
+        drop_pairs(ctx, *v);
     *kernel_out = cand[best];
     if (ms_out)
         for (int c = 0; c < 3; ++c)

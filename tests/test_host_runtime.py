@@ -33,3 +33,26 @@ def test_a_host_result_comes_from_one_loop_ordered_after_its_array(sim, answers,
     assert {p[0] for p in launches} == {hostsim.GATHER if answers[0] == 1000 else hostsim.SEGMENTS_UP}
     assert all(p[4] in ("-", "ok") for p in launches)
     assert len({p[2] for p in launches}) == (2 if views >= 8 else 1)
+
+
+@pytest.mark.parametrize("kw,loop,build", [({}, hostsim.SEGMENTS, "build_cells"),
+                                           (dict(kernel=L.KERNEL_PAIRS), hostsim.PAIRS, "build_pairs"),
+                                           (dict(volume_upsampling=2), hostsim.SEGMENTS_UP, "build_cells")])
+@pytest.mark.parametrize("host", [False, True])
+def test_an_array_whose_build_failed_is_not_kept(sim, kw, loop, build, host):
+    """The launch that fills a derived array fails once, after its allocation: the call
+    fails, or is served without the array where the gather loop can; the memory is given
+    back, and the next call builds the array before it reads it."""
+    v, _ = sim.volume()
+    used = sim.memory_used()
+    sim.clear()
+    sim.fail(build)
+    up = "volume_upsampling" in kw
+    assert sim.project(v, sim.settings(**kw), host=host) == (L.OK if up else L.ERR_CUDA)
+    assert {p[0] for p in sim.projections()} == ({hostsim.GATHER} if up else set())
+    assert sim.memory_used() == used
+    sim.clear()
+    assert sim.project(v, sim.settings(**kw), host=host) == L.OK
+    assert sim.record()[0].startswith(build) and sim.record()[0].endswith("done")
+    assert {(p[0], p[4]) for p in sim.projections()} == {(loop, "ok")}
+    assert sim.memory_used() > used
