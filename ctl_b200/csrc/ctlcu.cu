@@ -42,6 +42,7 @@ struct VolumeEntry {
     void* cells = nullptr;      // coefficient cells (CTLCU_KERNEL_CELLS), built on first use
     size_t cell_bytes = 0;
     uint32_t plan_refs = 0;     // plans that reference this volume (release is refused meanwhile)
+    bool replayed = false;      // captured launches, or a no-allocation call's, may read the derived arrays
     void* pairs = nullptr;      // x-pair array (CTLCU_KERNEL_PAIRS), built on first use
     size_t pair_bytes = 0;
     uint64_t handle = 0;        // 0 for the temporary volume of ctlcu_project_volume
@@ -514,6 +515,16 @@ int ensure_texture(ctlcu_ctx* ctx, VolumeEntry& v, int f, cudaTextureObject_t* o
     return CTLCU_OK;
 }
 
+bool is_capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
+
 // Whether an up-sampled projection reads the coefficient cells: they are built
 // already, or this call may build them.  The gather loop serves such calls without
 // any array, so one is built only where nothing else can miss the memory: no
@@ -523,12 +534,8 @@ bool cells_for_upsampling(ctlcu_ctx* ctx, VolumeEntry& v, bool may_build)
 {
     if (v.cells)
         return true;
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (!may_build || ctx->budget || cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess ||
-        capturing != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
+    if (!may_build || ctx->budget || is_capturing(ctx->stream))
         return false;
-    }
     const int n[3] = { (int)v.desc.n[0], (int)v.desc.n[1], (int)v.desc.n[2] };
     const CellLayout L = cell_layout(n);
     size_t free_bytes = 0, total = 0;
@@ -740,6 +747,8 @@ int project_device(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s_in, c
         if (r)
             return r;
     }
+    if (is_capturing(st))
+        v.replayed = true;
     job_args(a, s, V, M, C, R, derived_loop(mode));
     ViewGeom* geom = nullptr;
     CU_TRY(ctx, cudaMallocAsync((void**)&geom, sizeof(ViewGeom) * (size_t)V * M, st));
@@ -2109,12 +2118,14 @@ int ctlcu_autotune(ctlcu_ctx* ctx, uint64_t volume, const ctlcu_settings* settin
     if (r)
         return r;
     ctx->tuned[std::make_tuple(volume, channels, rows, n_modules)] = ctlcu_ctx::Tuned{ cand[best], shape_of(&bs) };
-    // keep only the array the chosen loop reads
+    // keep only the array the chosen loop reads, and those that replayed work may read
     cudaStreamSynchronize(ctx->stream);
-    if (cand[best] != CTLCU_KERNEL_CELLS)
-        drop_cells(ctx, *v);
-    if (cand[best] != CTLCU_KERNEL_PAIRS)
-        drop_pairs(ctx, *v);
+    if (!v->replayed && !v->plan_refs) {
+        if (cand[best] != CTLCU_KERNEL_CELLS)
+            drop_cells(ctx, *v);
+        if (cand[best] != CTLCU_KERNEL_PAIRS)
+            drop_pairs(ctx, *v);
+    }
     *kernel_out = cand[best];
     if (ms_out)
         for (int c = 0; c < 3; ++c)
@@ -2680,6 +2691,7 @@ int ctlcu_project_noalloc(ctlcu_ctx* ctx, uint64_t volume, const ctlcu_settings*
     r = order_after_staging(ctx, st);
     if (r)
         return r;
+    v->replayed = true;
     job_args(a, &eff, n_views, n_modules, channels, rows, derived_loop(mode));
     CU_TRY(ctx, launch_setup(pmats, n_views, n_modules, geom, nullptr, nullptr, ctx->d_flags, st));
     a.geom = geom;

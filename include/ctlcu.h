@@ -311,7 +311,8 @@ CTLCU_API int ctlcu_count_samples(ctlcu_ctx* ctx, uint64_t volume, const ctlcu_s
  * fields set in `settings` stay fixed.  The result serves later calls on this volume with the same
  * detector size and module count whose kernel is CTLCU_KERNEL_AUTO (loop and
  * shape) or the tuned loop (shape); only the derived array the winner reads is
- * kept.  *kernel receives the loop; ms_out (optional) the three loop times in
+ * kept, but for a volume that a plan, a call during stream capture or
+ * ctlcu_project_noalloc has read, which keeps all it has.  *kernel receives the loop; ms_out (optional) the three loop times in
  * ms (cells, pairs, gather) with the default shape.  pmats: host or device.
  */
 CTLCU_API int ctlcu_autotune(ctlcu_ctx* ctx, uint64_t volume, const ctlcu_settings* settings,
@@ -580,6 +581,8 @@ CTLCU_API int ctlcu_spectral_combine_noisy(ctlcu_ctx* ctx, const float* material
  *    mean-voxel volume, a texture) must exist already, built by an earlier
  *    ctlcu_project or ctlcu_autotune of this volume with these settings;
  *    otherwise CTLCU_ERR_INVALID_ARGUMENT names the missing one.
+ *    From this call on the volume keeps its derived arrays until it is
+ *    released, so that a captured call may be replayed.
  *  - The first call on a device looks up the scratch array's address there
  *    (cudaGetSymbolAddress); make that first call before any stream capture.
  *    The address is kept for the life of the process: after cudaDeviceReset

@@ -56,3 +56,44 @@ def test_an_array_whose_build_failed_is_not_kept(sim, kw, loop, build, host):
     assert sim.record()[0].startswith(build) and sim.record()[0].endswith("done")
     assert {(p[0], p[4]) for p in sim.projections()} == {(loop, "ok")}
     assert sim.memory_used() > used
+
+
+@pytest.mark.parametrize("reader", ["noalloc", "captured", "plan", "project"])
+@pytest.mark.parametrize("upsampling", [1, 2])
+def test_autotuning_leaves_arrays_that_captured_work_may_read(sim, reader, upsampling):
+    """A no-allocation call, a call during capture of its stream and a plan leave launches
+    behind that may be replayed for as long as the volume lives: autotuning, won by the
+    gather loop, does not free the cells that they read.  After a plain call it does."""
+    import ctypes as C
+    v, _ = sim.volume()
+    s = sim.settings(volume_upsampling=upsampling)
+    assert sim.project(v, s) == L.OK  # builds the cells
+    cells = sim.projections()[-1][3]
+    if reader == "noalloc":
+        assert sim.project(v, s, call="ctlcu_project_noalloc") == L.OK
+        assert sim.projections()[-1][3:5] == (cells, "ok")
+    elif reader == "captured":
+        sim.lib.sim_capturing(1)
+        assert sim.project(v, s) == L.OK
+        sim.lib.sim_capturing(0)
+        assert sim.projections()[-1][3] == cells
+    elif reader == "plan":
+        if upsampling != 1:
+            pytest.skip("plans take volumes as they are")
+        q = L.Request(v, sim.device(96), sim.device(256), 1, 1, 8, 8)
+        plan = C.c_void_p()
+        assert sim.lib.ctlcu_plan_create(sim.h, C.byref(q), 1, C.byref(s), C.byref(plan)) == L.OK
+    for loop in (hostsim.SEGMENTS, hostsim.PAIRS):
+        sim.lib.sim_mode_ms(loop, 9.0)
+    sim.lib.sim_mode_ms(hostsim.GATHER, 1.0)
+    loop = C.c_int()
+    assert sim.lib.ctlcu_autotune(sim.h, v, C.byref(sim.settings()), sim.device(96), 1, 1, 8, 8, 0, C.byref(loop),
+                                  None) == L.OK
+    assert loop.value == L.KERNEL_GATHER
+    freed = any(line == f"freed_array {cells}" for line in sim.record())
+    assert freed == (reader == "project")
+    sim.clear()
+    assert sim.project(v, sim.settings(volume_upsampling=2), call="ctlcu_project_noalloc") == L.OK
+    assert sim.projections()[0][4] == ("-" if freed else "ok")
+    if reader == "plan":
+        sim.lib.ctlcu_plan_destroy(plan)
