@@ -39,6 +39,7 @@ struct Alloc {
 struct Built {
     int stream;
     long at;
+    Clock reads;  // the last launch of each stream that read it
 };
 
 std::mutex mu;
@@ -144,7 +145,7 @@ const Alloc* find(const void* p)
     return (const char*)p < (const char*)it->first + (it->second.bytes ? it->second.bytes : 1) ? &it->second : nullptr;
 }
 
-void wrote(void* p, cudaStream_t s) { built[p] = { id_of(s), op(s) }; }
+void wrote(void* p, cudaStream_t s) { built[p] = { id_of(s), op(s), {} }; }
 
 // "-" without an array, "ok" after its build, "race" if nothing orders this stream after
 // the build, "stale" if it was freed or never built.
@@ -156,6 +157,7 @@ const char* read(const void* p, cudaStream_t s)
     if (it == built.end())
         return "stale";
     Clock& c = clocks[id_of(s)];
+    it->second.reads[id_of(s)] = c[id_of(s)];
     return c[it->second.stream] >= it->second.at ? "ok" : "race";
 }
 
@@ -350,6 +352,11 @@ cudaError_t cudaFreeAsync(void* p, cudaStream_t s)
 {
     LOCK;
     op(s);
+    auto it = built.find(p);
+    if (it != built.end())
+        for (const auto& r : it->second.reads)
+            if (clocks[id_of(s)][r.first] < r.second)
+                note("freed_while_read %p", p);
     return give(p);
 }
 cudaError_t cudaHostAlloc(void** p, size_t bytes, unsigned)

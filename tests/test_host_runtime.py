@@ -58,7 +58,7 @@ def test_an_array_whose_build_failed_is_not_kept(sim, kw, loop, build, host):
     assert sim.memory_used() > used
 
 
-@pytest.mark.parametrize("reader", ["noalloc", "captured", "plan", "project"])
+@pytest.mark.parametrize("reader", ["noalloc", "captured", "plan", "project", "stream"])
 @pytest.mark.parametrize("upsampling", [1, 2])
 def test_autotuning_leaves_arrays_that_captured_work_may_read(sim, reader, upsampling):
     """A no-allocation call, a call during capture of its stream and a plan leave launches
@@ -77,6 +77,9 @@ def test_autotuning_leaves_arrays_that_captured_work_may_read(sim, reader, upsam
         assert sim.project(v, s) == L.OK
         sim.lib.sim_capturing(0)
         assert sim.projections()[-1][3] == cells
+    elif reader == "stream":  # a plain call, still running on a stream of the caller's
+        assert sim.project(v, s, stream=sim.lib.sim_stream()) == L.OK
+        assert sim.projections()[-1][3:5] == (cells, "ok")
     elif reader == "plan":
         if upsampling != 1:
             pytest.skip("plans take volumes as they are")
@@ -91,9 +94,22 @@ def test_autotuning_leaves_arrays_that_captured_work_may_read(sim, reader, upsam
                                   None) == L.OK
     assert loop.value == L.KERNEL_GATHER
     freed = any(line == f"freed_array {cells}" for line in sim.record())
-    assert freed == (reader == "project")
+    assert freed == (reader in ("project", "stream")) and sim.count("freed_while_read") == 0
     sim.clear()
     assert sim.project(v, sim.settings(volume_upsampling=2), call="ctlcu_project_noalloc") == L.OK
     assert sim.projections()[0][4] == ("-" if freed else "ok")
     if reader == "plan":
         sim.lib.ctlcu_plan_destroy(plan)
+
+
+@pytest.mark.parametrize("upsampling", [2, 3])
+def test_an_upsampled_call_leaves_a_capture_elsewhere_alone(sim, upsampling):
+    """While another thread captures a stream of its own in the global mode, cudaMalloc
+    fails and ends that capture; an up-sampled call does not need it."""
+    v, _ = sim.volume()
+    sim.clear()
+    sim.lib.sim_foreign_capture(1)
+    assert sim.project(v, sim.settings(volume_upsampling=upsampling)) == L.OK
+    assert sim.lib.sim_unsafe_calls() == 0
+    assert {(p[0], p[4]) for p in sim.projections()} == {(hostsim.SEGMENTS_UP, "ok")}
+    sim.lib.sim_foreign_capture(0)
