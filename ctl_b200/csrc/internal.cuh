@@ -142,13 +142,16 @@ inline CellLayout cell_layout(const int n[3])
 
 // Bounds of the cells whose eight voxels are not all zero, behind the last cell: the
 // maxima over them of -x, x, -y, y, -z, z, -(x+y), x+y, -(x-y), x-y (cell indexes), or
-// kSupportNone; then kSupportNone, or 1 where a voxel is infinite or not a number.  Air around the object and the corners outside a scanner's circular
+// kSupportNone; then kSupportNone, or 1 where a voxel is wild: not a number, infinite, or
+// so large (kWild) that a cell's coefficients may overflow where its interpolant does not.
+// Air around the object and the corners outside a scanner's circular
 // field of view are exact zeros; a ray's samples there add nothing, so the cell
 // loops start and end at these slabs (the diagonal pairs make the outline an
 // octagon).  With cylinders of 90% of the volume's width: 256^3 -> 60 x 512^2 11.2 ->
 // 9.1 ms, 512^3 helical, 180 views, 2.15 -> 1.54 ms; volumes without zeros: 11.2 ->
 // 11.4 and 2.14 -> 2.17 ms.
-constexpr int kSupport = 11, kSupportNonFinite = 10;
+constexpr int kSupport = 11, kSupportWild = 10;
+constexpr double kWild = 5192296858534827628530496329220096.0;  // 2^112
 constexpr size_t kSupportBytes = 64;
 constexpr int kSupportNone = (int)0x80808080;  // a byte pattern: set by memset
 

@@ -1067,7 +1067,8 @@ __device__ __forceinline__ void store_patch(const ProjectArgs& a, uint32_t vm, u
 
 // One ray of the gather loop, up-sampled.  A voxel that is infinite or not a number
 // reaches a whole cell through the cell's polynomial, where the replicated grid holds
-// it to the samples next to that voxel: volumes with such voxels take this road.
+// it to the samples next to that voxel, and masks near the largest FP32 number overflow
+// its coefficients: volumes with such voxels (kWild) take this road.
 template <Accum ACC>
 __device__ __noinline__ void gather_upsampled(const ProjectArgs& a, const ViewGeom& g, double px, double py, bool live,
                                               Accumulator<ACC>& acc)
@@ -1109,8 +1110,8 @@ __device__ __forceinline__ void cells_item(const ProjectArgs& a, uint32_t b, uin
     const ViewGeom& g = a.geom[ok ? vm : 0u];
     const bool live = ok && g.valid;
     Accumulator<ACC> acc;
-    // (up-sampled volumes with voxels that are no numbers, see gather_upsampled)
-    const bool by_voxel = (M == Mode::CellsUp || M == Mode::SegmentsUp) && __ldg(a.support + kSupportNonFinite) > 0;
+    // (up-sampled volumes with wild voxels, see gather_upsampled)
+    const bool by_voxel = (M == Mode::CellsUp || M == Mode::SegmentsUp) && __ldg(a.support + kSupportWild) > 0;
     auto ray = [&](double px, double py) {
         if (by_voxel) {
             gather_upsampled<ACC>(a, g, px, py, live, acc);

@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(128)
     const uint32_t rows = (L.sz + L.sy - 1) / L.sy;  // the last one may be the pair's tail alone
     const uint32_t x = slot >> 1;
     int z_lo = INT_MAX, z_hi = -1, y_lo = INT_MAX, y_hi = -1;  // this thread's cells that are not zero
-    bool odd = false;  // a voxel is infinite or not a number
+    bool wild = false;  // a voxel is not below kWild
     const size_t ys = (size_t)ex, zs = (size_t)ex * ey;
     for (uint32_t p = blockIdx.z; p < pairs; p += gridDim.z) {
         const uint32_t z = 2 * p + (slot & 1u);
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(128)
                 const double a = to_float<T>(v[0]), b = to_float<T>(v[1]);
                 const double c = to_float<T>(v[zs]), d = to_float<T>(v[zs + 1]);
                 some = a != 0.0 || b != 0.0 || c != 0.0 || d != 0.0;
-                odd = odd || !isfinite(a) || !isfinite(b) || !isfinite(c) || !isfinite(d);
+                wild = wild || !(fabs(a) < kWild && fabs(b) < kWild && fabs(c) < kWild && fabs(d) < kWild);
                 const double l = a + b, lx = b - a, h = c + d, hx = d - c;
                 s = l + h;
                 sx = lx + hx;
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(128)
     const int xi = (int)x;
     const bool any = y_hi >= 0;
     const int m[kSupport] = { -xi, xi, -y_lo, y_hi, -z_lo, z_hi, -(xi + y_lo), xi + y_hi, -(xi - y_hi), xi - y_lo,
-                              odd ? 1 : kSupportNone };
+                              wild ? 1 : kSupportNone };
     for (int i = 0; i < kSupport; ++i) {
         const int w = __reduce_max_sync(0xffffffffu, any ? m[i] : kSupportNone);
         if ((threadIdx.x & 31u) == 0)

@@ -257,3 +257,28 @@ def test_upsampled_samples_are_placed_as_well_as_by_the_gather_loop(ctx, upsampl
             assert err[L.KERNEL_AUTO] <= err[L.KERNEL_GATHER]
     finally:
         v.release()
+
+
+@pytest.mark.parametrize("mask", [-3.4e38, 3.4e38, 1e34, np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("sampling", [0.05, 1.0])
+def test_upsampled_volumes_with_masks_give_what_the_gather_loop_gives(ctx, mask, sampling):
+    """Voxels masked with the largest numbers, infinities or NaN, next to each other along
+    an edge, a face and a diagonal: an up-sampled call gives the bits of the gather loop,
+    which interpolates between voxels and holds no sums over eight of them.  Finite
+    masks leave every sample, and an FP64 sum of them, finite."""
+    vol = _volume((23, 19, 21), 29)
+    for z, y, x in ((5, 5, 5), (5, 6, 6), (9, 9, 9), (9, 9, 10), (14, 12, 4), (15, 13, 5), (0, 0, 22)):
+        vol[z, y, x] = mask
+    C, R = 43, 31
+    P = _axis_views(C, R, 0.9, 0.29)
+    v = ctx.volume(VoxelVolume(vol, (0.3, 0.3, 0.3)))
+    try:
+        for accum in (L.ACCUM_FP64, L.ACCUM_KAHAN):
+            st = dict(ray_sampling=sampling, volume_upsampling=2, accum=accum)
+            want = ctx.project(v, P, C, R, Settings(kernel=L.KERNEL_GATHER, **st))
+            got = ctx.project(v, P, C, R, Settings(**st))
+            if np.isfinite(mask) and accum == L.ACCUM_FP64:
+                assert np.isfinite(want).all() and (np.abs(want) > 1e33).any()
+            np.testing.assert_array_equal(got, want)
+    finally:
+        v.release()
