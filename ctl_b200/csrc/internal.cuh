@@ -305,8 +305,8 @@ cudaError_t launch_average_samples(const float* in, uint32_t n_samples, uint64_t
 cudaError_t launch_combine_linear(const float* slope, const float* offset, const double* d_times, uint64_t per_view,
                                   uint32_t n_views, float* out, cudaStream_t s);
 cudaError_t launch_spectral(const float* proj, uint32_t n_materials, uint64_t per_view, uint32_t n_views,
-                            const float* mu, const double* intensity, const float* response, const int* skip,
-                            uint32_t n_bins, const double* total, float* out, cudaStream_t s);
+                            const float* mu, const double* intensity, const float* response, const int* live,
+                            uint32_t n_live, const double* total, float* out, cudaStream_t s);
 cudaError_t launch_saturation(float* data, uint32_t n_views, uint32_t n_modules, uint64_t ppm, int domain,
                               const ctlcu_saturation_model& model, const float* scale, cudaStream_t s);
 cudaError_t launch_spectral_noisy(const float* proj, uint32_t n_materials, uint32_t n_views, uint32_t n_modules,

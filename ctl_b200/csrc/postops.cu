@@ -316,35 +316,36 @@ __global__ void combine_kernel(const float* __restrict__ slope, const float* __r
 // intensity: [bin][view]; response: [bin] (1 without a detector response model).
 //
 // Bound by FP32 issue (about 13 instructions per bin and pixel, 8 of them the
-// exponential).  A block takes kSpectralPixels pixels of one view; its bins, without
-// the skipped ones, are laid out in shared memory once, and a thread combines
-// kSpectralPer pixels at a time, so a bin's values are read once for all of them and
-// their exponentials overlap.  The arithmetic of a pixel is the same as pixel by
-// pixel.  M: materials, 0 for any number (values of a pixel read from global memory in
-// every bin).  90 x 512^2, 2 materials, 30 bins: 2.09 ms with a thread per pixel
-// reading every bin's five values from global memory, 0.42 ms now.
-constexpr uint32_t kSpectralPer = 4, kSpectralThreads = 256, kSpectralPixels = kSpectralPer * kSpectralThreads;
-constexpr uint32_t kSpectralTable = 6144;  // floats of shared memory
+// exponential).  A block takes PER pixels per thread of one view; the values of the live
+// bins (those not skipped) are laid out in shared memory, as many at a time as fit, and
+// a bin's are read once for all pixels of a thread, whose exponentials overlap.  The
+// arithmetic of a pixel does not depend on PER or the block.  M: materials in registers,
+// 0 for any number (values of a pixel read from global memory in every bin).
+// 90 x 512^2, 2 materials, 30 bins: 2.09 ms with a thread per pixel reading every bin's
+// five values from global memory, 0.42 ms now.
+constexpr uint32_t kSpectralThreads = 256;
+constexpr uint32_t kSpectralPer = 4;                  // pixels per thread where that leaves no SM idle
+constexpr uint32_t kSpectralTable = 6144;             // most floats of shared memory
+constexpr uint32_t kSpectralFull = 148u * 4u;         // blocks of a job that fills the GPU
 
-template <int M>
+template <int M, int PER>
 __global__ void __launch_bounds__(kSpectralThreads)
     spectral_kernel(const float* __restrict__ proj, uint32_t n_materials, uint64_t per_view, uint32_t n_views,
                     const float* __restrict__ mu, const double* __restrict__ intensity,
-                    const float* __restrict__ response, const int* __restrict__ skip, uint32_t n_bins,
-                    const double* __restrict__ total, float* __restrict__ out)
+                    const float* __restrict__ response, const int* __restrict__ live, uint32_t n_live, uint32_t most,
+                    uint32_t width, const double* __restrict__ total, float* __restrict__ out)
 {
-    __shared__ float table[kSpectralTable];  // per bin: intensity, response, then mu of each material
-    __shared__ uint32_t bins_of[kSpectralTable / 3 + 1], held;
+    extern __shared__ float table[];  // per bin: intensity, response, then mu of each material, if width has room
     const uint64_t n = per_view * n_views;
-    const uint32_t width = 2u + (M ? (uint32_t)M : 0u), most = kSpectralTable / (width < 3u ? 3u : width);
+    const uint32_t threads = blockDim.x, mats = M ? (uint32_t)M : n_materials;
+    const uint64_t pixels = (uint64_t)PER * threads;
     for (uint32_t v = blockIdx.y; v < n_views; v += gridDim.y)
-        for (uint64_t first = blockIdx.x * (uint64_t)kSpectralPixels; first < per_view;
-             first += gridDim.x * (uint64_t)kSpectralPixels) {
-            uint64_t at[kSpectralPer];
-            float p[kSpectralPer][M ? M : 1], sum[kSpectralPer];
+        for (uint64_t first = blockIdx.x * pixels; first < per_view; first += gridDim.x * pixels) {
+            uint64_t at[PER];
+            float p[PER][M ? M : 1], sum[PER];
 #pragma unroll
-            for (uint32_t j = 0; j < kSpectralPer; ++j) {
-                const uint64_t i = first + threadIdx.x + j * kSpectralThreads;
+            for (int j = 0; j < PER; ++j) {
+                const uint64_t i = first + threadIdx.x + (uint64_t)j * threads;
                 at[j] = (uint64_t)v * per_view + (i < per_view ? i : per_view - 1);
                 sum[j] = 0.0f;
                 if (M)
@@ -352,48 +353,41 @@ __global__ void __launch_bounds__(kSpectralThreads)
                     for (int m = 0; m < M; ++m)
                         p[j][m] = proj[(uint64_t)m * n + at[j]];
             }
-            for (uint32_t b0 = 0; b0 < n_bins;) {
+            for (uint32_t b0 = 0; b0 < n_live; b0 += most) {
+                const uint32_t part = min(most, n_live - b0);
                 __syncthreads();
-                if (threadIdx.x == 0) {
-                    held = 0;
-                    uint32_t b = b0;
-                    for (; b < n_bins && held < most; ++b)
-                        if (!skip[b])
-                            bins_of[held++] = b;
-                    bins_of[most] = b;  // where the next part begins
+                for (uint32_t e = threadIdx.x; e < part * width; e += threads) {
+                    const uint32_t q = e / width, c = e - q * width;
+                    const uint64_t b = (uint64_t)live[b0 + q];
+                    table[e] = c == 0 ? (float)intensity[b * n_views + v]
+                                      : (c == 1 ? response[b] : mu[b * n_materials + (c - 2u)]);
                 }
                 __syncthreads();
-                const uint32_t live = held;
-                b0 = bins_of[most];
-                for (uint32_t e = threadIdx.x; e < live; e += kSpectralThreads) {
-                    const uint32_t b = bins_of[e];
-                    table[e * width] = (float)intensity[(uint64_t)b * n_views + v];
-                    table[e * width + 1] = response[b];
-                    if (M)
-                        for (int m = 0; m < M; ++m)
-                            table[e * width + 2 + m] = mu[(uint64_t)b * n_materials + m];
-                }
-                __syncthreads();
-                for (uint32_t e = 0; e < live; ++e) {
+                for (uint32_t e = 0; e < part; ++e) {
                     const float* t = table + e * width;
 #pragma unroll
-                    for (uint32_t j = 0; j < kSpectralPer; ++j) {
+                    for (int j = 0; j < PER; ++j) {
                         float x = 0.0f;
                         if (M) {
 #pragma unroll
                             for (int m = 0; m < M; ++m)
                                 x = fmaf(p[j][m], t[2 + m], x);
                         } else {
-                            for (uint32_t m = 0; m < n_materials; ++m)
-                                x = fmaf(proj[(uint64_t)m * n + at[j]], mu[(uint64_t)bins_of[e] * n_materials + m], x);
+                            if (width > 2u)
+                                for (uint32_t m = 0; m < mats; ++m)
+                                    x = fmaf(proj[(uint64_t)m * n + at[j]], t[2 + m], x);
+                            else
+                                for (uint32_t m = 0; m < mats; ++m)
+                                    x = fmaf(proj[(uint64_t)m * n + at[j]],
+                                             mu[(uint64_t)live[b0 + e] * n_materials + m], x);
                         }
                         sum[j] = fmaf(t[0] * expf(-x), t[1], sum[j]);
                     }
                 }
             }
 #pragma unroll
-            for (uint32_t j = 0; j < kSpectralPer; ++j)
-                if (first + threadIdx.x + j * kSpectralThreads < per_view)
+            for (int j = 0; j < PER; ++j)
+                if (first + threadIdx.x + (uint64_t)j * threads < per_view)
                     out[at[j]] = logf((float)total[v] / sum[j]);
         }
 }
@@ -532,22 +526,43 @@ cudaError_t launch_poisson_noise(float* data, uint32_t n_views, uint32_t n_modul
 }
 
 cudaError_t launch_spectral(const float* proj, uint32_t n_materials, uint64_t per_view, uint32_t n_views,
-                            const float* mu, const double* intensity, const float* response, const int* skip,
-                            uint32_t n_bins, const double* total, float* out, cudaStream_t s)
+                            const float* mu, const double* intensity, const float* response, const int* live,
+                            uint32_t n_live, const double* total, float* out, cudaStream_t s)
 {
     const uint64_t n = per_view * n_views;
     if (n == 0)
         return cudaSuccess;
-    const dim3 g((unsigned)std::min<uint64_t>((per_view + kSpectralPixels - 1) / kSpectralPixels, 1u << 20),
+    const uint32_t width = 2u + (n_materials <= kSpectralTable - 2u ? n_materials : 0u);
+    const uint32_t most = std::max(1u, std::min(kSpectralTable / width, n_live));
+    // Four pixels per thread where the materials are in registers, the blocks still fill the
+    // GPU and a view's last block wastes less than an eighth of its pixels, else one; and
+    // blocks that divide a view evenly.  Wall time of the call with four always, and now, us: 4096
+    // views of 64 pixels, 2 materials, 30 bins 245, 178; 2000 views of 1100 pixels, 4
+    // materials, 200 bins 961, 773; 9 materials, 200 bins, 4 views of 512^2 1598, 961.
+    const uint64_t wide = (uint64_t)kSpectralPer * kSpectralThreads, blocks = (per_view + wide - 1) / wide;
+    const bool four = n_materials <= 8 && blocks * n_views >= kSpectralFull && (blocks * wide - per_view) * 8 <= per_view;
+    const uint64_t ones = (per_view + kSpectralThreads - 1) / kSpectralThreads;  // blocks of one pixel per thread,
+    const uint32_t threads = (uint32_t)(((per_view + ones - 1) / ones + 31) / 32 * 32);  // of equal size
+    const uint64_t pixels = four ? wide : threads;
+    const dim3 g((unsigned)std::min<uint64_t>((per_view + pixels - 1) / pixels, 1u << 20),
                  std::min<uint32_t>(n_views, 65535u));
-#define CTLCU_SPECTRAL(M)                                                                                         \
-    spectral_kernel<M><<<g, kSpectralThreads, 0, s>>>(proj, n_materials, per_view, n_views, mu, intensity, response, \
-                                                      skip, n_bins, total, out)
+    const size_t smem = sizeof(float) * most * width;
+#define CTLCU_SPECTRAL(M)                                                                                          \
+    if (M && four)                                                                                                 \
+        spectral_kernel<M, M ? kSpectralPer : 1><<<g, kSpectralThreads, smem, s>>>(                                \
+            proj, n_materials, per_view, n_views, mu, intensity, response, live, n_live, most, width, total, out);        \
+    else                                                                                                           \
+        spectral_kernel<M, 1><<<g, threads, smem, s>>>(proj, n_materials, per_view, n_views, mu, intensity,        \
+                                                       response, live, n_live, most, width, total, out)
     switch (n_materials) {
     case 1: CTLCU_SPECTRAL(1); break;
     case 2: CTLCU_SPECTRAL(2); break;
     case 3: CTLCU_SPECTRAL(3); break;
     case 4: CTLCU_SPECTRAL(4); break;
+    case 5: CTLCU_SPECTRAL(5); break;
+    case 6: CTLCU_SPECTRAL(6); break;
+    case 7: CTLCU_SPECTRAL(7); break;
+    case 8: CTLCU_SPECTRAL(8); break;
     default: CTLCU_SPECTRAL(0); break;
     }
 #undef CTLCU_SPECTRAL

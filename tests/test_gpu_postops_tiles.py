@@ -63,3 +63,46 @@ def test_spectral_combine_matches_64_bits(ctx, materials, bins, views, per_view)
     want = np.log(np.float32(total).astype(np.float64)[:, None] / acc)
     bound = (bins + 16) * 2.0 ** -24 + 4.0 * 2.0 ** -24 * np.maximum(1.0, np.abs(want))
     assert (np.abs(out.cpu().numpy() - want) <= bound).all()
+
+
+@pytest.mark.parametrize("materials", [2, 8, 9])
+@pytest.mark.parametrize("bins,views,per_view", [(5, 300, 33), (5, 300, 1024), (5, 300, 1100), (9, 700, 64), (3, 2, 20000),
+                                                 (1200, 1, 257)])
+def test_spectral_combine_over_small_views_and_many_materials(ctx, materials, bins, views, per_view):
+    """Both numbers of pixels per thread, blocks of every size, materials in registers and
+    not, more bins than a table holds, every third bin skipped: the bound of the test above."""
+    test_spectral_combine_matches_64_bits(ctx, materials, bins, views, per_view)
+
+
+def test_spectral_combine_without_a_live_bin(ctx):
+    """No intensity in any bin: log(total / 0)."""
+    import torch
+    proj = torch.zeros((1, 2, 40), device="cuda")
+    out = torch.empty((2, 40), device="cuda")
+    mu, inten, total = np.ones((3, 1), np.float32), np.zeros((3, 2)), np.ones(2)
+    torch.cuda.synchronize()
+    ctx._check(ctx.lib.ctlcu_spectral_combine(
+        ctx.h, C.c_void_p(proj.data_ptr()), 1, 2, 40, C.c_void_p(mu.ctypes.data), C.c_void_p(inten.ctypes.data), None, 3,
+        C.c_void_p(total.ctypes.data), C.c_void_p(out.data_ptr()), None))
+    assert np.isposinf(out.cpu().numpy()).all()
+
+
+def test_spectral_combine_takes_more_materials_than_a_table_holds(ctx):
+    """6143 materials: the exponent is a chain of as many FP32 additions of positive terms,
+    within 6143 2^-24 of itself (0.5), which the logarithm passes on absolutely."""
+    import torch
+    M, bins, views, px = 6143, 2, 2, 40
+    rng = np.random.default_rng(3)
+    proj = rng.uniform(0.0, 1.0, (M, views, px)).astype(np.float32)
+    mu = rng.uniform(0.0, 2.0 / M, (bins, M)).astype(np.float32)
+    inten = rng.uniform(10.0, 1000.0, (bins, views))
+    total = inten.sum(0)
+    d = torch.from_numpy(proj).cuda()
+    out = torch.empty((views, px), device="cuda")
+    torch.cuda.synchronize()
+    ctx._check(ctx.lib.ctlcu_spectral_combine(
+        ctx.h, C.c_void_p(d.data_ptr()), M, views, px, C.c_void_p(mu.ctypes.data), C.c_void_p(inten.ctypes.data), None,
+        bins, C.c_void_p(total.ctypes.data), C.c_void_p(out.data_ptr()), None))
+    e = np.einsum("bm,mvp->bvp", mu.astype(np.float64), proj.astype(np.float64))
+    want = np.log(total[:, None] / (inten[:, :, None] * np.exp(-e)).sum(0))
+    assert np.abs(out.cpu().numpy() - want).max() <= 6143 * 2.0 ** -24 * e.max() + 1e-6
