@@ -175,11 +175,28 @@ __device__ float noisy_count(double lam, Stream& s)
 // at 1e5 photons: 661 -> 356 us (a queue per block, whose barriers its warps
 // waited at: 367).
 //
-// The tile is the largest, up to 1024 pixels, that still gives every SM 16 warps: few
-// pixels end up in partly filled rounds, while a small job keeps the GPU busy (2 x
-// 216 x 216: 30 us with tiles of 32, 63 with 1024, 32 before).
+// The tile is the largest, from 128 up to 1024 pixels, that still gives every SM 48 warps:
+// few pixels end up in partly filled rounds, while warps that finish early leave none idle
+// (360 views of 64 x 256 pixels, 5 and 1e5 photons: 130 and 163 us, 153 and 176 with 16
+// warps).  A job whose pixels all fit the GPU at one per thread is over when its slowest
+// pixel is, and takes them so (kNoiseSmall; 2 x 216 x 216, 300 photons: 27.2 us, 32.5 with
+// tiles of 32; 524288 pixels, more than fit: 51.3 us, 47.3 in tiles).
 constexpr uint32_t kNoiseTile = 1024;   // most pixels per warp
 constexpr uint32_t kNoiseWarps = 4;     // warps per block
+constexpr uint64_t kNoiseSmall = 148ull * 2048;
+
+__global__ void __launch_bounds__(128)
+    poisson_small_kernel(float* __restrict__ data, uint32_t total, uint32_t per_view, uint32_t ppm,
+                         const float* __restrict__ i0, uint32_t k0, uint32_t k1)
+{
+    const uint32_t i = blockIdx.x * 128u + threadIdx.x;
+    if (i >= total)
+        return;
+    const uint32_t view = i / per_view, pix = i - view * per_view;
+    const float i0m = i0[pix / ppm];
+    Stream s{ pix, view, 0u, k0, k1 };
+    data[i] = logf(i0m / noisy_count((double)i0m * exp(-(double)data[i]), s));
+}
 
 __global__ void __launch_bounds__(32 * kNoiseWarps)
     poisson_kernel(float* __restrict__ data, uint32_t n_views, uint32_t n_modules, uint32_t ppm,
@@ -515,8 +532,13 @@ cudaError_t launch_poisson_noise(float* data, uint32_t n_views, uint32_t n_modul
     if (total == 0)
         return cudaSuccess;
     const uint64_t per_view = (uint64_t)n_modules * ppm;
+    if (total <= kNoiseSmall) {
+        poisson_small_kernel<<<(unsigned)((total + 127) / 128), 128, 0, s>>>(
+            data, (uint32_t)total, (uint32_t)per_view, ppm, i0, (uint32_t)seed, (uint32_t)(seed >> 32));
+        return cudaGetLastError();
+    }
     uint32_t tile = kNoiseTile;
-    while (tile > 32u && total < 148ull * 16 * tile)
+    while (tile > 128u && total < 148ull * 48 * tile)
         tile /= 2;
     const uint64_t tiles = (per_view - 1) / tile + 1;
     const uint64_t blocks = std::min<uint64_t>((tiles * n_views + kNoiseWarps - 1) / kNoiseWarps, 148ull * 64);

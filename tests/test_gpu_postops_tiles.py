@@ -37,6 +37,15 @@ def test_noise_is_the_oracles_draw_for_draw(ctx, views, modules, ppm, photons):
     assert np.abs(got[~inf] - want[~inf]).max(initial=0.0) <= 2.0 ** -22 * max(1.0, np.abs(want[~inf]).max(initial=0.0))
 
 
+@pytest.mark.parametrize("views,modules,ppm", [(1, 1, 303104), (1, 1, 303105), (9800, 1, 31), (300, 1, 1023), (299, 1, 1025),
+                                               (70, 5, 911), (2, 64, 8000), (1, 1, 3637249)])
+@pytest.mark.parametrize("photons", [6.0, 3.0e3])
+def test_noise_of_larger_jobs_is_the_oracles_draw_for_draw(ctx, views, modules, ppm, photons):
+    """The largest job of one pixel per thread and the smallest of tiles, views that end
+    within a tile, tiles of 128, 256 and 512 pixels: the bar of the test above."""
+    test_noise_is_the_oracles_draw_for_draw(ctx, views, modules, ppm, photons)
+
+
 @pytest.mark.parametrize("materials", [1, 2, 4, 5])
 @pytest.mark.parametrize("bins,views,per_view", [(1, 1, 1), (7, 3, 1023), (33, 2, 1025), (2500, 2, 130)])
 def test_spectral_combine_matches_64_bits(ctx, materials, bins, views, per_view):
