@@ -654,6 +654,9 @@ bool derived_loop(Mode m)
 // neighbouring sub-rays, where one lane after the other would trace rays a whole pixel
 // apart from its neighbours' (320x320x256, 60 x 160 x 120, 2 x 2 rays: 7.1 -> 4.3 ms).
 // Other counts are traced one after the other; 3 rays a side would leave lanes idle.
+// The choice does not look at the number of views (launch_views divides what exceeds a
+// grid): sums across lanes and sums one after the other round differently, and a view
+// is the same in every call that holds it.
 void job_args(ProjectArgs& a, const ctlcu_settings* s, uint32_t V, uint32_t M, uint32_t C, uint32_t R, bool spread)
 {
     const LaunchShape sh = shape_of(s);
@@ -661,9 +664,9 @@ void job_args(ProjectArgs& a, const ctlcu_settings* s, uint32_t V, uint32_t M, u
     const uint32_t rx = s->rays_per_pixel[0], ry = s->rays_per_pixel[1];
     spread = spread && (rx == 1 || rx == 2 || rx == 4) && (ry == 1 || ry == 2 || ry == 4) && C < (1u << 28) &&
              R < (1u << 28);
-    if (spread) {  // block numbers stay well inside 32 bits
+    if (spread) {  // the block numbers of a chunk of view groups stay well inside 32 bits
         const uint64_t tiles = ((uint64_t)C * rx / tx + 1) * ((uint64_t)R * ry / ty + 1);
-        spread = tiles < (1u << 26) && tiles * V * M < (1u << 26);
+        spread = tiles < (1u << 26) && tiles * M < (1u << 26);
     }
     a.sub_x = spread ? log2u(rx) : 0u;
     a.sub_y = spread ? log2u(ry) : 0u;
@@ -688,6 +691,26 @@ void job_args(ProjectArgs& a, const ctlcu_settings* s, uint32_t V, uint32_t M, u
     a.wx_shift = log2u(tx / sh.lanes_x);
     a.tx_shift = log2u(tx);
     a.ty_shift = log2u(ty);
+}
+
+// The projection launch, in as many as keep each within a grid's 2^31 - 1 blocks.
+int launch_views(ctlcu_ctx* ctx, ProjectArgs a, Mode mode, Accum acc, int dtype, cudaStream_t st)
+{
+    const uint32_t V = a.n_views, views = 1u << a.vpb_shift;
+    const uint64_t per_group = (uint64_t)a.n_modules * a.tiles_per_vm;
+    const uint64_t most = std::min<uint64_t>(V, std::max<uint64_t>(1u, 0x7fffffffull / per_group) * views);
+    const ViewGeom* geom = a.geom;
+    float* out = a.out;
+    for (uint64_t v = 0; v < V; v += most) {
+        a.n_views = (uint32_t)std::min<uint64_t>(most, V - v);
+        a.n_vm = a.n_views * a.n_modules;
+        a.view_groups = (a.n_views + views - 1) / views;
+        a.geom = geom + v * a.n_modules;
+        a.out = out + v * a.n_modules * (size_t)a.rows * a.channels;
+        CU_TRY(ctx, launch_project(a, mode, acc, dtype, st));
+        ++ctx->launches;
+    }
+    return CTLCU_OK;
 }
 
 VolumeEntry* find_volume(ctlcu_ctx* ctx, uint64_t h)
@@ -763,10 +786,10 @@ int project_device(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s_in, c
     a.out = d_out;
     a.flags = ctx->d_flags;
     a.counter = nullptr;
-    CU_TRY(ctx, launch_project(a, mode, (Accum)s->accum, dtype, st));
-    ctx->launches += 2;
+    ++ctx->launches;
+    r = launch_views(ctx, a, mode, (Accum)s->accum, dtype, st);
     CU_TRY(ctx, cudaFreeAsync(geom, st));
-    return CTLCU_OK;
+    return r;
 }
 
 // Views per chunk of a projection into host memory: five equal chunks, then
@@ -1079,7 +1102,7 @@ struct BatchDevice {
 // Validate the requests and, when the settings select the cell kernel, build
 // the per-request launch arguments (building cell arrays as needed).
 int prepare_batch(ctlcu_ctx* ctx, const ctlcu_request* requests, uint32_t n, const ctlcu_settings* s,
-                  BatchPrep& bp)
+                  bool persistent, BatchPrep& bp)
 {
     for (uint32_t i = 0; i < n; ++i) {
         const ctlcu_request& q = requests[i];
@@ -1103,6 +1126,17 @@ int prepare_batch(ctlcu_ctx* ctx, const ctlcu_request* requests, uint32_t n, con
     const ctlcu_settings eff = resolve_kernel(ctx, *find_volume(ctx, requests[0].volume), s, requests[0].channels,
                                               requests[0].rows, requests[0].n_modules);
     bp.shape = shape_of(&eff);
+    // all work items in 31 bits, and the persistent launch's warps in 32 with room for the
+    // counter to run past; a lane for every sub-ray only where that holds
+    const uint64_t most = persistent ? std::min<uint64_t>(0x7fffffffull, (0xffffffffull - (1ull << 20)) / (bp.shape.block / 32))
+                                     : 0x7fffffffull;
+    uint64_t spread_items = 0;
+    for (uint32_t i = 0; i < n; ++i) {
+        ProjectArgs a = {};
+        job_args(a, &eff, requests[i].n_views, requests[i].n_modules, requests[i].channels, requests[i].rows, true);
+        spread_items += std::min<uint64_t>((uint64_t)a.view_groups * a.n_modules * a.tiles_per_vm, 1ull << 40);
+    }
+    const bool spread = spread_items <= most;
     uint64_t vm = 0, items = 0;
     for (uint32_t i = 0; i < n; ++i) {
         const ctlcu_request& q = requests[i];
@@ -1115,7 +1149,7 @@ int prepare_batch(ctlcu_ctx* ctx, const ctlcu_request* requests, uint32_t n, con
         if (mode != Mode::Cells && mode != Mode::Segments && mode != Mode::Pairs)
             return fail(ctx, CTLCU_ERR_INVALID_ARGUMENT, "request %u does not take the cell kernel", i);
         bp.mode = mode;
-        job_args(br.a, &eff, q.n_views, q.n_modules, q.channels, q.rows, true);
+        job_args(br.a, &eff, q.n_views, q.n_modules, q.channels, q.rows, spread);
         br.a.out = q.out;
         br.a.flags = ctx->d_flags;
         br.a.counter = nullptr;
@@ -1626,7 +1660,7 @@ int ctlcu_project_batch(ctlcu_ctx* ctx, const ctlcu_request* requests, uint32_t 
     cudaSetDevice(ctx->device);
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
     BatchPrep bp;
-    r = prepare_batch(ctx, requests, n_requests, settings, bp);
+    r = prepare_batch(ctx, requests, n_requests, settings, false, bp);
     if (r == CTLCU_OK)
         r = order_after_staging(ctx, st);
     if (r)
@@ -1788,7 +1822,7 @@ int ctlcu_plan_create_form(ctlcu_ctx* ctx, const ctlcu_request* requests, uint32
         return fail(ctx, CTLCU_ERR_OUT_OF_MEMORY, "plan allocation failed");
     p->ctx = ctx;
     p->settings = *settings;
-    r = prepare_batch(ctx, requests, n_requests, settings, p->bp);
+    r = prepare_batch(ctx, requests, n_requests, settings, true, p->bp);
     if (r == CTLCU_OK && !p->bp.persistent)
         r = fail(ctx, CTLCU_ERR_INVALID_ARGUMENT,
                  "plans need the cell kernel (software trilinear, volumeUpSampling 1)");
@@ -2706,9 +2740,8 @@ int ctlcu_project_noalloc(ctlcu_ctx* ctx, uint64_t volume, const ctlcu_settings*
     a.out = out;
     a.flags = ctx->d_flags;
     a.counter = nullptr;
-    CU_TRY(ctx, launch_project(a, mode, (Accum)eff.accum, dtype, st));
-    ctx->launches += 2;
-    return CTLCU_OK;
+    ++ctx->launches;
+    return launch_views(ctx, a, mode, (Accum)eff.accum, dtype, st);
 }
 
 }  // extern "C"

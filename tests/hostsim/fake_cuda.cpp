@@ -169,6 +169,11 @@ const char* read(const void* p, cudaStream_t s)
 SIM void sim_reset()
 {
     LOCK;
+    for (const auto& m : allocs)
+        munmap(const_cast<void*>(m.first), m.second.bytes ? m.second.bytes : 1);
+    allocs.clear();
+    built.clear();
+    used = 0;
     failures.clear();
     free_answers.clear();
     mode_ms.clear();

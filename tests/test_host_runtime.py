@@ -113,3 +113,44 @@ def test_an_upsampled_call_leaves_a_capture_elsewhere_alone(sim, upsampling):
     assert sim.lib.sim_unsafe_calls() == 0
     assert {(p[0], p[4]) for p in sim.projections()} == {(hostsim.SEGMENTS_UP, "ok")}
     sim.lib.sim_foreign_capture(0)
+
+
+@pytest.mark.parametrize("kernel", [L.KERNEL_CELLS, L.KERNEL_PAIRS])
+def test_sub_rays_get_lanes_whatever_the_number_of_views(sim, kernel):
+    """A view's sub-rays are summed across lanes, or one after the other, which rounds
+    differently: the choice goes by the detector alone, so that a view is the same in a
+    call of any length, in a chunk of a host result and in a no-allocation call.  Every
+    launch keeps its blocks within a grid's limit."""
+    v, _ = sim.volume()
+    s = sim.settings(rays_per_pixel=(4, 4), kernel=kernel)
+    sim.lib.sim_capacity(1 << 45)
+    C, R = 1024, 1024
+    tiles = (4 * C // 16) * (4 * R // 8)
+    for views, kw in ((1, {}), (600, {}), (40000, {}), (600, dict(host=True)), (600, dict(call="ctlcu_project_noalloc"))):
+        sim.clear()
+        assert sim.project(v, s, views=views, channels=C, rows=R, **kw) == L.OK
+        launches = sim.projections()
+        assert {p[5] for p in launches} == {(2, 2)} and sum(p[1] for p in launches) == views
+        assert all((p[1] + 1) // 2 * tiles <= 0x7fffffff for p in launches)
+
+
+@pytest.mark.parametrize("form", [L.PLAN_PERSISTENT, L.PLAN_GRIDS])
+@pytest.mark.parametrize("requests,lanes", [(40, (2, 2)), (500, (0, 0))])
+def test_a_batch_too_large_with_a_lane_per_sub_ray_goes_without(sim, form, requests, lanes):
+    """500 views of 1024^2 with 4 x 4 rays a pixel: with a lane for every ray their warps do
+    not fit the 32 bits of the persistent launch's counter, one after the other they do."""
+    import ctypes as C
+    v, _ = sim.volume()
+    s = sim.settings(rays_per_pixel=(4, 4))
+    q = (L.Request * requests)()
+    pm, out = sim.device(96 * 24), sim.device(4 * 24 << 20)
+    for r in q:
+        r.volume, r.pmats, r.out, r.n_views, r.n_modules, r.channels, r.rows = v, pm, out, 24, 1, 1024, 1024
+    plan = C.c_void_p()
+    assert sim.lib.ctlcu_plan_create_form(sim.h, q, requests, C.byref(s), form, C.byref(plan)) == L.OK, sim.error()
+    if form == L.PLAN_GRIDS:
+        assert {p[5] for p in sim.projections()} == {lanes}
+    sim.lib.ctlcu_plan_destroy(plan)
+    sim.clear()
+    assert sim.lib.ctlcu_project_batch(sim.h, q, requests, C.byref(s), None) == L.OK
+    assert {p[5] for p in sim.projections()} == {(2, 2)}  # one grid per request: these fit
