@@ -1227,24 +1227,29 @@ __global__ void __maxnreg__(CTLCU_GATHER_MAXREG) project_kernel(const __grid_con
     const ViewGeom& g = a.geom[ok ? vm : 0u];
     const bool live = ok && g.valid;
     Accumulator<ACC> acc;
-    const double ix = 1.0 / a.rays_x, iy = 1.0 / a.rays_y;
-    for (uint32_t rx = 0; rx < a.rays_x; ++rx)
-        for (uint32_t ry = 0; ry < a.rays_y; ++ry) {
-            const double px = (double)x - 0.5 + 0.5 * ix + rx * ix;
-            const double py = (double)y - 0.5 + 0.5 * iy + ry * iy;
-            Ray r = setup_ray<M>(a, g, px, py, live ? a.flags : nullptr);
-            if (!live)
-                r.n = 0;
-            if (M == Mode::Trilinear)
-                march_trilinear<T, ACC, UP>(a, r, acc);
-            else if (M == Mode::Nearest)
-                march_nearest<T, ACC>(a, r, acc);
-            else if (M == Mode::NearestSamples)
-                march_nearest_samples<T, ACC>(a, r, acc);
-            else
-                march_texture<ACC>(a, r, acc);
-        }
-    const float val = static_cast<float>(a.increment * acc.value() / (double)(a.rays_x * a.rays_y));
+    float val = 0.0f;
+    // the windows of march_nearest are the whole warp's; a lane without a ray stays out of
+    // the other loops
+    if (M == Mode::Nearest || live) {
+        const double ix = 1.0 / a.rays_x, iy = 1.0 / a.rays_y;
+        for (uint32_t rx = 0; rx < a.rays_x; ++rx)
+            for (uint32_t ry = 0; ry < a.rays_y; ++ry) {
+                const double px = (double)x - 0.5 + 0.5 * ix + rx * ix;
+                const double py = (double)y - 0.5 + 0.5 * iy + ry * iy;
+                Ray r = setup_ray<M>(a, g, px, py, live ? a.flags : nullptr);
+                if (!live)
+                    r.n = 0;
+                if (M == Mode::Trilinear)
+                    march_trilinear<T, ACC, UP>(a, r, acc);
+                else if (M == Mode::Nearest)
+                    march_nearest<T, ACC>(a, r, acc);
+                else if (M == Mode::NearestSamples)
+                    march_nearest_samples<T, ACC>(a, r, acc);
+                else
+                    march_texture<ACC>(a, r, acc);
+            }
+        val = static_cast<float>(a.increment * acc.value() / (double)(a.rays_x * a.rays_y));
+    }
     store_patch<false>(a, vm, x, y, val, ok);
 }
 
