@@ -563,8 +563,7 @@ int volume_args(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, Project
 {
     const bool interp = s->interpolate != 0;
     const int f = interp ? (int)s->volume_upsampling : 1;  // no interpolation forces f = 1
-    const Mode nearest = s->ray_sampling <= kNearestSegmentMaxSampling ? Mode::Nearest : Mode::NearestSamples;
-    mode = !interp ? nearest : (s->interp_mode == CTLCU_INTERP_TEXTURE ? Mode::Texture : Mode::Trilinear);
+    mode = !interp ? Mode::Nearest : (s->interp_mode == CTLCU_INTERP_TEXTURE ? Mode::Texture : Mode::Trilinear);
     const ctlcu_volume_desc& d = v.desc;
     float voxel[3];
     a.tex = 0;
@@ -640,6 +639,13 @@ int volume_args(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, Project
         a.corner_v[k] = a.corner[k] / a.voxel[k];
     }
     return CTLCU_OK;
+}
+
+// The nearest-voxel loop for this job (other loops as they are).
+Mode loop_for_job(Mode m, const ctlcu_settings* s, uint32_t V, uint32_t M, uint32_t C, uint32_t R)
+{
+    const uint64_t rays = (uint64_t)V * M * C * R;  // at least; sub-rays of a pixel follow each other
+    return m == Mode::Nearest && s->ray_sampling > nearest_segment_max_sampling(rays) ? Mode::NearestSamples : m;
 }
 
 bool derived_loop(Mode m)
@@ -778,6 +784,7 @@ int project_device(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s_in, c
     }
     if (is_capturing(st))
         v.replayed = true;
+    mode = loop_for_job(mode, s, V, M, C, R);
     job_args(a, s, V, M, C, R, derived_loop(mode));
     ViewGeom* geom = nullptr;
     CU_TRY(ctx, cudaMallocAsync((void**)&geom, sizeof(ViewGeom) * (size_t)V * M, st));
@@ -2734,6 +2741,7 @@ int ctlcu_project_noalloc(ctlcu_ctx* ctx, uint64_t volume, const ctlcu_settings*
     if (r)
         return r;
     v->replayed = true;
+    mode = loop_for_job(mode, &eff, n_views, n_modules, channels, rows);
     job_args(a, &eff, n_views, n_modules, channels, rows, derived_loop(mode));
     CU_TRY(ctx, launch_setup(pmats, n_views, n_modules, geom, nullptr, nullptr, ctx->d_flags, st));
     a.geom = geom;

@@ -270,9 +270,18 @@ constexpr float kSegmentMaxSampling = 0.6f;
 constexpr float kSegmentUpMaxSampling = 1.0f / 6.0f;
 
 // The nearest-voxel loop goes by segments up to this ray_sampling, above it sample by
-// sample in FP64.  Segments / samples, ms, 256^3 -> 15 x 512^2: 0.3 3.2 / 7.4, 0.75 2.78
-// / 3.10, 0.9 2.66 / 2.62, 1.0 2.56 / 2.38.
-constexpr float kNearestSegmentMaxSampling = 0.8f;
+// sample.  Segments are fewer, but each waits for the one before, while samples follow
+// from FP64 positions of their own: a GPU filled with rays gains from segments at almost
+// any step, a few rays only at fine ones.  Segments / samples, us:
+//   64^2 rays through 256^3          0.3 296 / 340, 0.5 271 / 228, 0.75 244 / 164
+//   4 x 160^2 rays through 256^3     0.5 172 / 185, 0.6 167 / 160, 0.75 164 / 135
+//   24 x 512^2 rays through 256^3    0.6 4411 / 5945, 0.75 4221 / 4827, 0.8 4130 / 4543
+//   4 x 512^2 rays through 384^3     0.75 1262 / 1270, 0.8 1266 / 1198
+// Both sum in FP64, so that a view is the same in calls of any size.
+inline float nearest_segment_max_sampling(uint64_t rays)
+{
+    return rays < 148ull * 256 ? 0.4f : rays < 148ull * 2048 ? 0.55f : 0.75f;
+}
 
 // Launchers (raycast.cu / setup.cu / volume.cu).  All asynchronous on `s`.
 cudaError_t launch_batch_setup(const BatchSetup* reqs, uint32_t n_reqs, uint32_t total, ViewGeom* geom,

@@ -58,10 +58,11 @@ template <>
 struct Accumulator<Accum::F64> {
     double s = 0.0;
     __device__ __forceinline__ void add(float v) { s += static_cast<double>(v); }
-    __device__ __forceinline__ void add_product(float m, float v, float&)
+    __device__ __forceinline__ void add_product(float m, float v)
     {
         s = fma(static_cast<double>(m), static_cast<double>(v), s);
     }
+    __device__ __forceinline__ void add_product(float m, float v, float&) { add_product(m, v); }
     __device__ __forceinline__ void flush(float) {}
     __device__ __forceinline__ double value() const { return s; }
 };
@@ -799,10 +800,12 @@ __device__ __noinline__ uint2 nearest_run(const ProjectArgs& a, const Ray& r, in
 // elsewhere (about one segment in 10^4 at the default step).  The first and the last
 // sample of the reference's range lie outside the volume, or on its face, and are
 // taken on their own.  256^3 -> 45 x 512^2: 22.0 ms with every sample in FP64, 9.5
-// ms by segments.  An FP64 accumulator takes every voxel's m v exactly, as it takes
-// every sample in the other form; the others take two voxels' FP32 sum.
-template <typename T, Accum ACC>
-__device__ __forceinline__ void march_nearest(const ProjectArgs& a, const Ray& r, Accumulator<ACC>& acc)
+// ms by segments.  The sum is FP64's: m v is exact in it, and so, unless the voxels'
+// magnitudes differ by 2^20 and more, is the sum, whatever its order.  Both forms then give
+// the same bits, and the choice between them can go by the size of the job (30 views: 6.20
+// ms, 6.04 with Kahan sums of two voxels' FP32 sums).
+template <typename T>
+__device__ __forceinline__ void march_nearest(const ProjectArgs& a, const Ray& r, Accumulator<Accum::F64>& acc)
 {
     const T* __restrict__ vol = static_cast<const T*>(a.vol);
     if (r.n > 0)
@@ -842,7 +845,6 @@ __device__ __forceinline__ void march_nearest(const ProjectArgs& a, const Ray& r
             const float last = (float)(stop - at - 1);
             float k = 0.0f;
             do {
-                float part = 0.0f;
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
                     const float2 vxy = __ffma2_rn(make_float2(k, k), dxy, fr.bxy);
@@ -868,13 +870,12 @@ __device__ __forceinline__ void march_nearest(const ProjectArgs& a, const Ray& r
                         m = (float)run.y;
                     }
                     if (left >= 0.0f) {
-                        acc.add_product(m, load_voxel(vol + idx), part);
+                        acc.add_product(m, load_voxel(vol + idx));
                     } else {
                         m = 0.0f;
                     }
                     k += m;
                 }
-                acc.flush(part);
             } while (k <= last);
             advance_axis(fr.bxy.x, fr.mxy.x, dxy.x, lx, k);
             advance_axis(fr.bxy.y, fr.mxy.y, dxy.y, ly, k);
@@ -888,9 +889,9 @@ __device__ __forceinline__ void march_nearest(const ProjectArgs& a, const Ray& r
 }
 
 // The same, every sample on its own: the faster form where a voxel holds hardly more
-// than one (kNearestSegmentMaxSampling).
-template <typename T, Accum ACC>
-__device__ __forceinline__ void march_nearest_samples(const ProjectArgs& a, const Ray& r, Accumulator<ACC>& acc)
+// than one, or few rays leave each waiting for its segments (nearest_segment_max_sampling).
+template <typename T>
+__device__ __forceinline__ void march_nearest_samples(const ProjectArgs& a, const Ray& r, Accumulator<Accum::F64>& acc)
 {
     const T* __restrict__ vol = static_cast<const T*>(a.vol);
     for (int k = 0; k < r.n; ++k)
@@ -1239,12 +1240,12 @@ __global__ void __maxnreg__(CTLCU_GATHER_MAXREG) project_kernel(const __grid_con
                 Ray r = setup_ray<M>(a, g, px, py, live ? a.flags : nullptr);
                 if (!live)
                     r.n = 0;
-                if (M == Mode::Trilinear)
+                if constexpr (M == Mode::Trilinear)
                     march_trilinear<T, ACC, UP>(a, r, acc);
-                else if (M == Mode::Nearest)
-                    march_nearest<T, ACC>(a, r, acc);
-                else if (M == Mode::NearestSamples)
-                    march_nearest_samples<T, ACC>(a, r, acc);
+                else if constexpr (M == Mode::Nearest)
+                    march_nearest<T>(a, r, acc);
+                else if constexpr (M == Mode::NearestSamples)
+                    march_nearest_samples<T>(a, r, acc);
                 else
                     march_texture<ACC>(a, r, acc);
             }
@@ -1322,8 +1323,9 @@ cudaError_t launch_acc(const ProjectArgs& a, Mode mode, int dtype, dim3 grid, cu
     case Mode::Trilinear:
         return a.up != 1 ? launch_typed<Mode::Trilinear, ACC, true>(a, dtype, grid, s)
                          : launch_typed<Mode::Trilinear, ACC, false>(a, dtype, grid, s);
-    case Mode::Nearest: return launch_typed<Mode::Nearest, ACC, false>(a, dtype, grid, s);
-    case Mode::NearestSamples: return launch_typed<Mode::NearestSamples, ACC, false>(a, dtype, grid, s);
+    // their sums are FP64's whatever the accumulator (march_nearest)
+    case Mode::Nearest: return launch_typed<Mode::Nearest, Accum::F64, false>(a, dtype, grid, s);
+    case Mode::NearestSamples: return launch_typed<Mode::NearestSamples, Accum::F64, false>(a, dtype, grid, s);
     case Mode::Texture:
         project_kernel<float, Mode::Texture, ACC, false><<<grid, a.block, 0, s>>>(a);
         return cudaGetLastError();

@@ -61,6 +61,7 @@ typedef enum {
     CTLCU_ACCUM_FP64 = 0,  /* double accumulator, as raycasterprojector_interp.cl:48,66 */
     CTLCU_ACCUM_KAHAN = 1, /* float with compensated (Kahan) summation (default) */
     CTLCU_ACCUM_FP32 = 2   /* plain float */
+    /* without interpolation every one of them sums in double */
 } ctlcu_accum;
 
 /*

@@ -145,3 +145,34 @@ def test_fp64_accumulator_sums_the_samples_without_fp32_rounding(ctx, storage, s
         assert (err <= 1.2e-7 * np.abs(want) + 1e-12 * total)[~ties].all()
     finally:
         v.release()
+
+
+@pytest.mark.parametrize("storage", [L.F32, L.F16])
+@pytest.mark.parametrize("sampling", [0.3, 0.4, 0.5, 0.7, 0.75, 0.76])
+def test_a_view_is_the_same_in_calls_of_any_size(ctx, storage, sampling):
+    """The loop goes by the number of rays: a view alone (segments up to 0.4), in a call
+    of 48 thousand rays (up to 0.55) and of 338 thousand (up to 0.75), on the device and in
+    chunks into host memory, has the same bits, with any accumulator."""
+    import torch
+    vol = np.random.default_rng(31).uniform(0.01, 0.05, (33, 37, 41)).astype(np.float32)
+    if storage == L.F16:
+        vol = vol.astype(np.float16).astype(np.float32)
+    C, R, V = 72, 67, 70
+    P = G.circular_flat(V, 300.0, 600.0, G.FlatDetector(C, R, 1.1, 1.1), rng=np.random.default_rng(1), jitter_mm=0.5,
+                        tilt_deg=0.2)
+    assert C * R < 148 * 256 <= 10 * C * R < 148 * 2048 <= V * C * R
+    v = ctx.volume(VoxelVolume(vol, (1.0, 1.1, 1.2)), storage)
+    try:
+        for accum in (L.ACCUM_KAHAN, L.ACCUM_FP64, L.ACCUM_FP32):
+            st = Settings(ray_sampling=sampling, interpolate=False, accum=accum)
+            whole = ctx.project(v, P, C, R, st)
+            for n in (1, 10):
+                np.testing.assert_array_equal(ctx.project(v, P[20:20 + n].copy(), C, R, st), whole[20:20 + n])
+            out = torch.empty(whole.shape, device="cuda")
+            ctx.project(v, torch.from_numpy(P).cuda(), C, R, st, out=out)
+            ctx.sync()
+            np.testing.assert_array_equal(out.cpu().numpy(), whole)
+        want, _ = oracle.project_fp64(vol, (1.0, 1.1, 1.2), P[:3], C, R, ray_sampling=sampling, interpolate=False)
+        assert rel_err(whole[:3], want).max() <= 1e-4
+    finally:
+        v.release()
