@@ -43,6 +43,7 @@ struct VolumeEntry {
     size_t cell_bytes = 0;
     bool cells_pooled = false;  // in pool memory
     uint32_t plan_refs = 0;     // plans that reference this volume (release is refused meanwhile)
+    UpLoop up = UpLoop::Ask;    // how up-sampled calls are to read it
     bool replayed = false;      // captured launches, or a no-allocation call's, may read the derived arrays
     void* pairs = nullptr;      // x-pair array (CTLCU_KERNEL_PAIRS), built on first use
     size_t pair_bytes = 0;
@@ -527,6 +528,18 @@ bool is_capturing(cudaStream_t st)
     return status != cudaStreamCaptureStatusNone;
 }
 
+// Whether the current device has the room for the cells of `times` such volumes that
+// up-sampled calls build: a quarter of its free memory.
+bool room_for_cells(const ctlcu_volume_desc& d, uint32_t times)
+{
+    const int n[3] = { (int)d.n[0], (int)d.n[1], (int)d.n[2] };
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) == cudaSuccess && cell_layout(n).count * kCellBytes * times <= free_bytes / 4)
+        return true;
+    cudaGetLastError();
+    return false;
+}
+
 // Whether an up-sampled projection reads the coefficient cells: they are built
 // already, or this call may build them.  The gather loop serves such calls without
 // any array, so one is built only where nothing else can miss the memory: no
@@ -538,17 +551,12 @@ bool is_capturing(cudaStream_t st)
 // another stream's capture in the global mode, which cudaMalloc would break, goes on.
 bool cells_for_upsampling(ctlcu_ctx* ctx, VolumeEntry& v, bool may_build)
 {
+    if (v.up == UpLoop::Gather)
+        return false;
     if (v.cells)
         return true;
-    if (!may_build || ctx->budget || is_capturing(ctx->stream))
+    if (!may_build || ctx->budget || is_capturing(ctx->stream) || (v.up == UpLoop::Ask && !room_for_cells(v.desc, 1)))
         return false;
-    const int n[3] = { (int)v.desc.n[0], (int)v.desc.n[1], (int)v.desc.n[2] };
-    const CellLayout L = cell_layout(n);
-    size_t free_bytes = 0, total = 0;
-    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || L.count * kCellBytes > free_bytes / 4) {
-        cudaGetLastError();
-        return false;
-    }
     if (ensure_cells(ctx, v, true) == CTLCU_OK)
         return true;
     cudaGetLastError();
@@ -1365,6 +1373,60 @@ int transform(ctlcu_ctx* ctx, float* data, uint32_t n_views, uint64_t per_view, 
 
 }  // namespace
 
+int ctlcu::project_volume(ctlcu_ctx* ctx, const ctlcu_volume_desc* desc, const float* volume,
+                          const ctlcu_settings* settings, const double* pmats, uint32_t n_views, uint32_t n_modules,
+                          uint32_t channels, uint32_t rows, float* out, UpLoop up)
+{
+    TraceRange trace_("ctlcu_project_volume");
+    if (!ctx)
+        return CTLCU_ERR_INVALID_ARGUMENT;
+    std::lock_guard<std::mutex> lk(ctx->mu);
+    if (!volume || !pmats || !out)
+        return fail(ctx, CTLCU_ERR_INVALID_ARGUMENT, "volume, pmats or out is NULL");
+    int r = check_desc(ctx, desc);
+    if (r)
+        return r;
+    r = check_settings(ctx, settings);
+    if (r)
+        return r;
+    r = check_job(ctx, n_views, n_modules, channels, rows);
+    if (r)
+        return r;
+    cudaSetDevice(ctx->device);
+    r = check_local(ctx, { volume, pmats, out });
+    if (r)
+        return r;
+    if (ctx->cache_max && !is_device_ptr(volume)) {
+        // a host volume seen before (same description and content) is projected
+        // from its resident copy: no upload, no cell build
+        VolumeEntry* cv = nullptr;
+        r = cached_volume(ctx, desc, volume, &cv);
+        if (r)
+            return r;
+        cv->up = up;
+        r = project_any(ctx, *cv, settings, pmats, n_views, n_modules, channels, rows, out, ctx->stream, true);
+        cv->up = UpLoop::Ask;
+        return r;
+    }
+    VolumeEntry v;
+    v.up = up;
+    r = make_volume(ctx, desc, volume, is_device_ptr(volume), true, v);
+    if (r == CTLCU_OK)
+        r = project_any(ctx, v, settings, pmats, n_views, n_modules, channels, rows, out, ctx->stream, true);
+    free_volume(ctx, v);
+    cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    if (r == CTLCU_OK && e != cudaSuccess)
+        r = fail(ctx, CTLCU_ERR_CUDA, "projection failed: %s", cudaGetErrorString(e));
+    return r;
+}
+
+bool ctlcu::upsampled_reads_cells(ctlcu_ctx* ctx, const ctlcu_volume_desc* desc, uint32_t times)
+{
+    std::lock_guard<std::mutex> lk(ctx->mu);
+    cudaSetDevice(ctx->device);
+    return !ctx->budget && room_for_cells(*desc, times);
+}
+
 extern "C" {
 
 int ctlcu_abi_version(void) { return CTLCU_ABI_VERSION; }
@@ -1613,43 +1675,7 @@ int ctlcu_project_volume(ctlcu_ctx* ctx, const ctlcu_volume_desc* desc, const fl
                          const ctlcu_settings* settings, const double* pmats, uint32_t n_views,
                          uint32_t n_modules, uint32_t channels, uint32_t rows, float* out)
 {
-    TraceRange trace_("ctlcu_project_volume");
-    if (!ctx)
-        return CTLCU_ERR_INVALID_ARGUMENT;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    if (!volume || !pmats || !out)
-        return fail(ctx, CTLCU_ERR_INVALID_ARGUMENT, "volume, pmats or out is NULL");
-    int r = check_desc(ctx, desc);
-    if (r)
-        return r;
-    r = check_settings(ctx, settings);
-    if (r)
-        return r;
-    r = check_job(ctx, n_views, n_modules, channels, rows);
-    if (r)
-        return r;
-    cudaSetDevice(ctx->device);
-    r = check_local(ctx, { volume, pmats, out });
-    if (r)
-        return r;
-    if (ctx->cache_max && !is_device_ptr(volume)) {
-        // a host volume seen before (same description and content) is projected
-        // from its resident copy: no upload, no cell build
-        VolumeEntry* cv = nullptr;
-        r = cached_volume(ctx, desc, volume, &cv);
-        if (r == CTLCU_OK)
-            r = project_any(ctx, *cv, settings, pmats, n_views, n_modules, channels, rows, out, ctx->stream, true);
-        return r;
-    }
-    VolumeEntry v;
-    r = make_volume(ctx, desc, volume, is_device_ptr(volume), true, v);
-    if (r == CTLCU_OK)
-        r = project_any(ctx, v, settings, pmats, n_views, n_modules, channels, rows, out, ctx->stream, true);
-    free_volume(ctx, v);
-    cudaError_t e = cudaStreamSynchronize(ctx->stream);
-    if (r == CTLCU_OK && e != cudaSuccess)
-        r = fail(ctx, CTLCU_ERR_CUDA, "projection failed: %s", cudaGetErrorString(e));
-    return r;
+    return project_volume(ctx, desc, volume, settings, pmats, n_views, n_modules, channels, rows, out, UpLoop::Ask);
 }
 
 int ctlcu_project_batch(ctlcu_ctx* ctx, const ctlcu_request* requests, uint32_t n_requests,

@@ -12,8 +12,10 @@
 // disjoint slice of the caller's host output, so there is no exchange between
 // the devices at all.  A view's result does not depend on the device or the
 // block it is computed in, so the output equals a single-device call bit for
-// bit.
+// bit.  Up-sampled volumes are read from their cells where there is room for
+// these, which differs from device to device: the group asks them all first.
 #include "ctlcu.h"
+#include "internal.cuh"
 
 #include <cuda_runtime.h>
 
@@ -177,11 +179,17 @@ int ctlcu_group_project_volume(ctlcu_group* g, const ctlcu_volume_desc* desc, co
     ctlcu_split_views(n_views, used, first.data());
     const size_t pm_per_view = (size_t)n_modules * 12;
     const size_t out_per_view = (size_t)n_modules * rows * channels;
+    ctlcu::UpLoop up = ctlcu::UpLoop::Cells;
+    for (uint32_t i = 0; i < used && settings->volume_upsampling > 1; ++i) {
+        const auto times = std::count(g->devices.begin(), g->devices.begin() + used, g->devices[i]);
+        if (!ctlcu::upsampled_reads_cells(g->ctxs[i], desc, (uint32_t)times))
+            up = ctlcu::UpLoop::Gather;
+    }
     std::vector<int> status(used, CTLCU_OK);
     auto run = [&](uint32_t i) {
         const uint32_t v0 = first[i], n = first[i + 1] - first[i];
-        status[i] = ctlcu_project_volume(g->ctxs[i], desc, volume, settings, pmats + v0 * pm_per_view, n, n_modules,
-                                         channels, rows, out + v0 * out_per_view);
+        status[i] = ctlcu::project_volume(g->ctxs[i], desc, volume, settings, pmats + v0 * pm_per_view, n, n_modules,
+                                          channels, rows, out + v0 * out_per_view, up);
     };
     if (used == 1) {
         run(0);

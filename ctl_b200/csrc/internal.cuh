@@ -283,6 +283,17 @@ inline float nearest_segment_max_sampling(uint64_t rays)
     return rays < 148ull * 256 ? 0.4f : rays < 148ull * 2048 ? 0.55f : 0.75f;
 }
 
+// How an up-sampled call reads its volume: the context asks for the room for the cells, or
+// the caller has (a device group, whose devices have to take the same loop).
+enum class UpLoop : int { Ask = 0, Cells = 1, Gather = 2 };
+
+// ctlcu_project_volume with that choice; and whether `times` such calls at once on the
+// context's device would read the cells (ctlcu.cu).
+int project_volume(ctlcu_ctx* ctx, const ctlcu_volume_desc* desc, const float* volume, const ctlcu_settings* settings,
+                   const double* pmats, uint32_t n_views, uint32_t n_modules, uint32_t channels, uint32_t rows,
+                   float* out, UpLoop up);
+bool upsampled_reads_cells(ctlcu_ctx* ctx, const ctlcu_volume_desc* desc, uint32_t times);
+
 // Launchers (raycast.cu / setup.cu / volume.cu).  All asynchronous on `s`.
 cudaError_t launch_batch_setup(const BatchSetup* reqs, uint32_t n_reqs, uint32_t total, ViewGeom* geom,
                                int* flags, cudaStream_t s);

@@ -15,7 +15,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(os.path.dirname(HERE))
 CSRC = os.path.join(ROOT, "ctl_b200", "csrc")
 CUDA = os.path.join(os.path.dirname(os.path.dirname(os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc"))), "include")
-UNITS = ("ctlcu", "hostcopy", "den", "nrrd")  # the ones without kernels
+UNITS = ("ctlcu", "group", "hostcopy", "den", "nrrd")  # the ones without kernels
 
 # loops (enum class Mode)
 GATHER, NEAREST, CELLS, PAIRS, SEGMENTS, CELLS_UP, SEGMENTS_UP = 0, 1, 3, 4, 5, 6, 7
@@ -40,7 +40,7 @@ class Sim:
     def __init__(self, path: str):
         self.lib = lib = C.CDLL(path)
         for name, res, args in L.SIGNATURES:
-            fn = getattr(lib, name, None)  # groups are not built
+            fn = getattr(lib, name, None)  # the geometry encoder is not built
             if fn is not None:
                 fn.restype, fn.argtypes = res, args
         lib.sim_record.restype = C.c_char_p
@@ -50,6 +50,7 @@ class Sim:
         lib.sim_used.restype = C.c_uint64
         lib.sim_capacity.argtypes = [C.c_uint64]
         lib.sim_mode_ms.argtypes = [C.c_int, C.c_float]
+        lib.sim_free_of_device.argtypes = [C.c_int, C.c_uint64]
         lib.sim_reset()
         self.h = C.c_void_p()
         assert lib.ctlcu_create(0, C.byref(self.h)) == L.OK

@@ -34,7 +34,7 @@ void merge(Clock& to, const Clock& from)
 
 struct Alloc {
     size_t bytes;
-    bool pooled;
+    int device;
 };
 struct Built {
     int stream;
@@ -58,7 +58,8 @@ uint64_t capacity = 180ull << 30, used = 0;
 int capturing = 0, capture_mode = 0, foreign_capture = 0, unsafe_calls = 0;
 int last_mode = 0;
 long next_handle = 16;
-int current = 0;
+thread_local int current = 0;
+std::map<int, uint64_t> free_of_device;     // what cudaMemGetInfo answers there, where set
 
 void note(const char* fmt, ...)
 {
@@ -115,7 +116,7 @@ cudaError_t take(void** p, size_t bytes, bool pooled)
     void* m = mmap(nullptr, bytes ? bytes : 1, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);
     if (m == MAP_FAILED)
         return cudaErrorMemoryAllocation;
-    allocs[m] = { bytes, pooled };
+    allocs[m] = { bytes, current };
     used += bytes;
     *p = m;
     return cudaSuccess;
@@ -176,6 +177,7 @@ SIM void sim_reset()
     used = 0;
     failures.clear();
     free_answers.clear();
+    free_of_device.clear();
     mode_ms.clear();
     record.clear();
     capacity = 180ull << 30;
@@ -186,6 +188,7 @@ SIM void sim_clear_record() { LOCK; record.clear(); }
 SIM void sim_capacity(uint64_t bytes) { LOCK; capacity = bytes; }
 SIM uint64_t sim_used() { LOCK; return used; }
 SIM void sim_free_answers(const uint64_t* v, int n) { LOCK; free_answers.assign(v, v + n); }
+SIM void sim_free_of_device(int device, uint64_t bytes) { LOCK; free_of_device[device] = bytes; }
 SIM void sim_fail(const char* what, int nth) { LOCK; failures[what] = nth; }
 SIM void sim_mode_ms(int mode, float ms) { LOCK; mode_ms[mode] = ms; }
 SIM void sim_capturing(int on) { LOCK; capturing = on; }
@@ -314,8 +317,8 @@ cudaError_t launch_transform(float*, uint64_t, uint32_t, const double*, bool, cu
 
 extern "C" {
 
-cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
-cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetDeviceCount(int* n) { *n = 2; return cudaSuccess; }
+cudaError_t cudaSetDevice(int d) { current = d; return cudaSuccess; }
 cudaError_t cudaGetDevice(int* d) { *d = current; return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "simulated"; }
@@ -384,6 +387,8 @@ cudaError_t cudaMemGetInfo(size_t* f, size_t* t)
     LOCK;
     *t = capacity;
     *f = used < capacity ? capacity - used : 0;
+    if (free_of_device.count(current))
+        *f = free_of_device[current];
     if (!free_answers.empty()) {
         *f = free_answers.front();
         free_answers.erase(free_answers.begin());
@@ -394,8 +399,9 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p)
 {
     LOCK;
     memset(a, 0, sizeof *a);
-    a->device = current;
-    a->type = find(p) ? cudaMemoryTypeDevice : pinned.count(p) ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;
+    const Alloc* m = find(p);
+    a->device = m ? m->device : current;
+    a->type = m ? cudaMemoryTypeDevice : pinned.count(p) ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;
     return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t st)

@@ -154,3 +154,32 @@ def test_a_batch_too_large_with_a_lane_per_sub_ray_goes_without(sim, form, reque
     sim.clear()
     assert sim.lib.ctlcu_project_batch(sim.h, q, requests, C.byref(s), None) == L.OK
     assert {p[5] for p in sim.projections()} == {(2, 2)}  # one grid per request: these fit
+
+
+@pytest.mark.parametrize("devices,free,loop", [
+    ((0, 1), (1 << 40, 1 << 40), hostsim.SEGMENTS_UP), ((0, 1), (1 << 40, 1000), hostsim.GATHER),
+    ((0, 1), (1000, 1 << 40), hostsim.GATHER), ((0, 1), (1000, 1000), hostsim.GATHER),
+    ((0, 0), (1 << 40, 0), hostsim.SEGMENTS_UP), ((0, 0), (1600000, 0), hostsim.GATHER)])
+@pytest.mark.parametrize("views", [2, 33])
+def test_a_group_projects_all_its_views_with_one_loop(sim, devices, free, loop, views):
+    """Whether an up-sampled volume's cells are built goes by the free memory, which
+    differs from device to device: the group decides once for all its devices, as the
+    result has to be a one-device call's bit for bit.  (A 16^3 volume's cells take 277
+    KB, a quarter of 1.6 MB holds one context's and not two.)"""
+    import ctypes as C
+    import numpy as np
+    for d, f in enumerate(free):
+        sim.lib.sim_free_of_device(d, f)
+    g = C.c_void_p()
+    assert sim.lib.ctlcu_group_create((C.c_int * 2)(*devices), 2, C.byref(g)) == L.OK
+    vol, P, out = np.zeros(16 ** 3, np.float32), np.zeros(12 * views), np.zeros(64 * views, np.float32)
+    for up in (2, 1, 2):
+        sim.clear()
+        s = sim.settings(volume_upsampling=up)
+        assert sim.lib.ctlcu_group_project_volume(g, C.byref(sim.desc((16, 16, 16))), vol.ctypes.data, C.byref(s),
+                                                  P.ctypes.data, views, 1, 8, 8, out.ctypes.data) == L.OK
+        launches = sim.projections()
+        assert sum(p[1] for p in launches) == views
+        assert {p[0] for p in launches} == ({loop} if up == 2 else {hostsim.SEGMENTS})
+        assert {p[4] for p in launches} <= {"ok", "-"}
+    assert sim.lib.ctlcu_group_destroy(g) == L.OK
