@@ -42,6 +42,7 @@ struct VolumeEntry {
     void* cells = nullptr;      // coefficient cells (CTLCU_KERNEL_CELLS), built on first use
     size_t cell_bytes = 0;
     bool cells_pooled = false;  // in pool memory
+    bool cells_optional = false;  // only up-sampled calls have read them, which run without
     uint32_t plan_refs = 0;     // plans that reference this volume (release is refused meanwhile)
     UpLoop up = UpLoop::Ask;    // how up-sampled calls are to read it
     bool replayed = false;      // captured launches, or a no-allocation call's, may read the derived arrays
@@ -288,42 +289,14 @@ int check_job(ctlcu_ctx* ctx, uint32_t V, uint32_t M, uint32_t C, uint32_t R)
     return CTLCU_OK;
 }
 
-// Upload (or device-copy) `data` into a new zero-padded volume in the storage dtype.
-int make_volume(ctlcu_ctx* ctx, const ctlcu_volume_desc* d, const float* data, bool on_device,
-                bool pooled, VolumeEntry& v)
+bool is_capturing(cudaStream_t st)
 {
-    const int n[3] = { (int)d->n[0], (int)d->n[1], (int)d->n[2] };
-    const size_t padded = (size_t)(n[0] + 2 * kPad) * (n[1] + 2 * kPad) * (n[2] + 2 * kPad);
-    const size_t bytes = padded * dtype_size(d->dtype);
-    if (ctx->budget && ctx->used + bytes > ctx->budget)
-        return fail(ctx, CTLCU_ERR_OUT_OF_MEMORY,
-                    "volume of %zu bytes exceeds the memory budget (%llu of %llu bytes used)", bytes,
-                    (unsigned long long)ctx->used, (unsigned long long)ctx->budget);
-    v.desc = *d;
-    v.bytes = bytes;
-    v.pooled = pooled;
-    if (pooled)
-        CU_TRY(ctx, cudaMallocAsync(&v.data, bytes, ctx->stream));
-    else
-        CU_TRY(ctx, cudaMalloc(&v.data, bytes));
-    const size_t nbytes = (size_t)n[0] * n[1] * n[2] * sizeof(float);
-    const float* src = data;
-    float* staging = nullptr;
-    if (!on_device) {
-        CU_TRY(ctx, cudaMallocAsync((void**)&staging, nbytes, ctx->stream));
-        if (nbytes >= HostCopier::kLeast && pageable(data) && ctx->copier.ensure() == cudaSuccess)
-            CU_TRY(ctx, ctx->copier.run(ctx->device, { { staging, const_cast<float*>(data), nbytes, nullptr } }, false,
-                                        ctx->stream));
-        else
-            CU_TRY(ctx, cudaMemcpyAsync(staging, data, nbytes, cudaMemcpyHostToDevice, ctx->stream));
-        src = staging;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
     }
-    CU_TRY(ctx, launch_pad_convert(src, v.data, n, d->dtype, ctx->stream));
-    ++ctx->launches;
-    if (staging)
-        CU_TRY(ctx, cudaFreeAsync(staging, ctx->stream));
-    ctx->used += bytes;
-    return CTLCU_OK;
+    return status != cudaStreamCaptureStatusNone;
 }
 
 // Frees the volume's coefficient cells (pair entries), if it has any.
@@ -351,6 +324,76 @@ void drop_pairs(ctlcu_ctx* ctx, VolumeEntry& v)
     ctx->used -= std::min<uint64_t>(ctx->used, v.pair_bytes);
     v.pairs = nullptr;
     v.pair_bytes = 0;
+}
+
+// Frees the cells that only up-sampled calls read and no replayed work may; true if any.
+bool reclaim(ctlcu_ctx* ctx)
+{
+    if (is_capturing(ctx->stream))
+        return false;
+    bool any = false;
+    for (auto& kv : ctx->vols) {
+        VolumeEntry& v = kv.second;
+        if (!v.cells || !v.cells_optional || v.replayed || v.plan_refs)
+            continue;
+        if (!any)
+            cudaDeviceSynchronize();  // calls on other streams may still read them
+        drop_cells(ctx, v);
+        any = true;
+    }
+    cudaMemPool_t pool;
+    if (any && cudaStreamSynchronize(ctx->stream) == cudaSuccess &&
+        cudaDeviceGetDefaultMemPool(&pool, ctx->device) == cudaSuccess)
+        cudaMemPoolTrimTo(pool, 0);
+    return any;
+}
+
+// Device memory, of its own or (`pooled`) of the stream-ordered pool; what only speeds up
+// other calls makes room for it.
+cudaError_t allocate(ctlcu_ctx* ctx, void** p, size_t bytes, bool pooled, cudaStream_t st)
+{
+    auto once = [&]() { return pooled ? cudaMallocAsync(p, bytes, st) : cudaMalloc(p, bytes); };
+    cudaError_t e = once();
+    if (e == cudaErrorMemoryAllocation && reclaim(ctx)) {
+        cudaGetLastError();
+        e = once();
+    }
+    return e;
+}
+
+// Upload (or device-copy) `data` into a new zero-padded volume in the storage dtype.
+int make_volume(ctlcu_ctx* ctx, const ctlcu_volume_desc* d, const float* data, bool on_device,
+                bool pooled, VolumeEntry& v)
+{
+    const int n[3] = { (int)d->n[0], (int)d->n[1], (int)d->n[2] };
+    const size_t padded = (size_t)(n[0] + 2 * kPad) * (n[1] + 2 * kPad) * (n[2] + 2 * kPad);
+    const size_t bytes = padded * dtype_size(d->dtype);
+    if (ctx->budget && ctx->used + bytes > ctx->budget)
+        return fail(ctx, CTLCU_ERR_OUT_OF_MEMORY,
+                    "volume of %zu bytes exceeds the memory budget (%llu of %llu bytes used)", bytes,
+                    (unsigned long long)ctx->used, (unsigned long long)ctx->budget);
+    v.desc = *d;
+    v.bytes = bytes;
+    v.pooled = pooled;
+    CU_TRY(ctx, allocate(ctx, &v.data, bytes, pooled, ctx->stream));
+    const size_t nbytes = (size_t)n[0] * n[1] * n[2] * sizeof(float);
+    const float* src = data;
+    float* staging = nullptr;
+    if (!on_device) {
+        CU_TRY(ctx, allocate(ctx, (void**)&staging, nbytes, true, ctx->stream));
+        if (nbytes >= HostCopier::kLeast && pageable(data) && ctx->copier.ensure() == cudaSuccess)
+            CU_TRY(ctx, ctx->copier.run(ctx->device, { { staging, const_cast<float*>(data), nbytes, nullptr } }, false,
+                                        ctx->stream));
+        else
+            CU_TRY(ctx, cudaMemcpyAsync(staging, data, nbytes, cudaMemcpyHostToDevice, ctx->stream));
+        src = staging;
+    }
+    CU_TRY(ctx, launch_pad_convert(src, v.data, n, d->dtype, ctx->stream));
+    ++ctx->launches;
+    if (staging)
+        CU_TRY(ctx, cudaFreeAsync(staging, ctx->stream));
+    ctx->used += bytes;
+    return CTLCU_OK;
 }
 
 void free_volume(ctlcu_ctx* ctx, VolumeEntry& v)
@@ -410,10 +453,7 @@ int ensure_cells(ctlcu_ctx* ctx, VolumeEntry& v, bool pooled)
         return fail(ctx, CTLCU_ERR_OUT_OF_MEMORY,
                     "cell array of %zu bytes exceeds the memory budget (%llu of %llu bytes used)", bytes,
                     (unsigned long long)ctx->used, (unsigned long long)ctx->budget);
-    if (pooled)
-        CU_TRY(ctx, cudaMallocAsync(&v.cells, bytes, ctx->stream));
-    else
-        CU_TRY(ctx, cudaMalloc(&v.cells, bytes));
+    CU_TRY(ctx, allocate(ctx, &v.cells, bytes, pooled, ctx->stream));
     v.cells_pooled = pooled;
     v.cell_bytes = bytes;
     ctx->used += bytes;
@@ -438,10 +478,7 @@ int ensure_pairs(ctlcu_ctx* ctx, VolumeEntry& v)
         return fail(ctx, CTLCU_ERR_OUT_OF_MEMORY,
                     "pair array of %zu bytes exceeds the memory budget (%llu of %llu bytes used)", bytes,
                     (unsigned long long)ctx->used, (unsigned long long)ctx->budget);
-    if (v.pooled)
-        CU_TRY(ctx, cudaMallocAsync(&v.pairs, bytes, ctx->stream));
-    else
-        CU_TRY(ctx, cudaMalloc(&v.pairs, bytes));
+    CU_TRY(ctx, allocate(ctx, &v.pairs, bytes, v.pooled, ctx->stream));
     v.pair_bytes = bytes;
     ctx->used += bytes;
     const cudaError_t e = launch_build_pairs(v.data, n, v.desc.dtype, L, v.pairs, ctx->stream);
@@ -518,16 +555,6 @@ int ensure_texture(ctlcu_ctx* ctx, VolumeEntry& v, int f, cudaTextureObject_t* o
     return CTLCU_OK;
 }
 
-bool is_capturing(cudaStream_t st)
-{
-    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
-        cudaGetLastError();
-        return true;
-    }
-    return status != cudaStreamCaptureStatusNone;
-}
-
 // Whether the current device has the room for the cells of `times` such volumes that
 // up-sampled calls build: a quarter of its free memory.
 bool room_for_cells(const ctlcu_volume_desc& d, uint32_t times)
@@ -557,8 +584,10 @@ bool cells_for_upsampling(ctlcu_ctx* ctx, VolumeEntry& v, bool may_build)
         return true;
     if (!may_build || ctx->budget || is_capturing(ctx->stream) || (v.up == UpLoop::Ask && !room_for_cells(v.desc, 1)))
         return false;
-    if (ensure_cells(ctx, v, true) == CTLCU_OK)
+    if (ensure_cells(ctx, v, true) == CTLCU_OK) {
+        v.cells_optional = true;
         return true;
+    }
     cudaGetLastError();
     ctx->err.clear();
     return false;
@@ -618,6 +647,7 @@ int volume_args(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, Project
         int r = ensure_cells(ctx, v, v.pooled);
         if (r)
             return r;
+        v.cells_optional = v.cells_optional && f > 1;
         // Up-sampled, the gather loop spends its time on the integer divisions from
         // grid to stored voxels and on eight loads a sample (101x97x89, f = 3, 60 x
         // 512 x 384: 88.6 ms against 6.6 from the cells).
@@ -865,7 +895,7 @@ int project_any(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, const d
         d_pm = pm_tmp;
     }
     if (!out_dev)
-        CU_TRY(ctx, cudaMallocAsync((void**)&d_out, out_bytes, st));
+        CU_TRY(ctx, allocate(ctx, (void**)&d_out, out_bytes, true, st));
     int r = CTLCU_OK;
     if (out_dev) {
         r = project_device(ctx, v, s, d_pm, V, M, C, R, d_out, st);

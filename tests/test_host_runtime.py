@@ -183,3 +183,35 @@ def test_a_group_projects_all_its_views_with_one_loop(sim, devices, free, loop, 
         assert {p[0] for p in launches} == ({loop} if up == 2 else {hostsim.SEGMENTS})
         assert {p[4] for p in launches} <= {"ok", "-"}
     assert sim.lib.ctlcu_group_destroy(g) == L.OK
+
+
+@pytest.mark.parametrize("what", ["volume", "result", "cells", "pairs"])
+@pytest.mark.parametrize("held", [False, True])
+def test_memory_that_only_speeds_up_is_given_back_when_it_is_needed(sim, what, held):
+    """Cells that up-sampled calls built (they run without) do not stand in the way of what
+    a call needs: a new volume, a result, another loop's array.  Cells that replayed work
+    may read stay, and so do those that a loop cannot do without."""
+    a, _ = sim.volume((40, 40, 40))
+    needed, _ = sim.volume((16, 16, 16))
+    assert sim.project(needed, sim.settings()) == L.OK
+    assert sim.project(a, sim.settings(volume_upsampling=2)) == L.OK
+    cells = sim.projections()[-1][3]
+    b, _ = sim.volume((30, 30, 30))
+    if held:
+        assert sim.project(a, sim.settings(volume_upsampling=2), call="ctlcu_project_noalloc") == L.OK
+    sim.lib.sim_capacity(sim.lib.sim_used() + 20000)
+    used = sim.memory_used()
+    sim.clear()
+    if what == "volume":
+        rc = sim.volume((30, 30, 30))[1]
+    elif what == "result":
+        rc = sim.project(needed, sim.settings(), views=100, channels=100, rows=30, host=True)
+    else:
+        rc = sim.project(b, sim.settings(kernel=L.KERNEL_PAIRS if what == "pairs" else L.KERNEL_CELLS))
+    assert rc == (L.ERR_OUT_OF_MEMORY if held else L.OK), sim.error()
+    freed = [line.split()[1] for line in sim.record() if line.startswith("freed_array")]
+    assert freed == ([] if held else [cells]) and sim.count("freed_while_read") == 0
+    assert sim.memory_used() == used if held else sim.memory_used() != used
+    sim.clear()
+    assert sim.project(a, sim.settings(volume_upsampling=2)) == L.OK
+    assert sim.projections()[-1][4] == ("ok" if held else "-")
