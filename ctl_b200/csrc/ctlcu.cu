@@ -381,11 +381,12 @@ int make_volume(ctlcu_ctx* ctx, const ctlcu_volume_desc* d, const float* data, b
     float* staging = nullptr;
     if (!on_device) {
         CU_TRY(ctx, allocate(ctx, (void**)&staging, nbytes, true, ctx->stream));
-        if (nbytes >= HostCopier::kLeast && pageable(data) && ctx->copier.ensure() == cudaSuccess)
-            CU_TRY(ctx, ctx->copier.run(ctx->device, { { staging, const_cast<float*>(data), nbytes, nullptr } }, false,
-                                        ctx->stream));
-        else
+        if (nbytes >= HostCopier::kLeast && pageable(data) && ctx->copier.ensure() == cudaSuccess) {
+            const HostCopyPart part = { staging, const_cast<float*>(data), nbytes, nullptr };
+            CU_TRY(ctx, ctx->copier.run(ctx->device, &part, 1, false, ctx->stream));
+        } else {
             CU_TRY(ctx, cudaMemcpyAsync(staging, data, nbytes, cudaMemcpyHostToDevice, ctx->stream));
+        }
         src = staging;
     }
     CU_TRY(ctx, launch_pad_convert(src, v.data, n, d->dtype, ctx->stream));
@@ -837,6 +838,8 @@ int project_device(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s_in, c
     return r;
 }
 
+constexpr size_t kMostChunks = 8;
+
 // Views per chunk of a projection into host memory: five equal chunks, then
 // chunks of 4/47, 2/47 and 1/47 of the views (8, 4, 2, 1 parts of 47), so
 // that the copy that follows the last kernel is of about 2% of the output.  A
@@ -908,8 +911,10 @@ int project_any(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, const d
         // A copy into pageable memory returns only when it is done: all chunks are
         // launched first and several threads copy behind them (a 256^3 host volume,
         // 30 x 512^2 into host memory: 14.0 -> 7.7 ms, with the upload's threads).
+        const std::vector<uint32_t> sizes = host_chunks(V);
         const bool threads = out_bytes >= HostCopier::kLeast && pageable(out) && ctx->copier.ensure() == cudaSuccess;
-        std::vector<HostCopyPart> parts;
+        HostCopyPart parts[kMostChunks];
+        size_t n_parts = 0;
         if (!ctx->copy_stream)
             CU_TRY(ctx, cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
         if (!ctx->aux_stream)
@@ -927,7 +932,6 @@ int project_any(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, const d
         CU_TRY(ctx, cudaEventRecord(ctx->order, st));
         CU_TRY(ctx, cudaStreamWaitEvent(ctx->aux_stream, ctx->order, 0));
         const cudaStream_t lanes[2] = { st, ctx->aux_stream };
-        const std::vector<uint32_t> sizes = host_chunks(V);
         const size_t view_values = (size_t)M * R * C;
         uint32_t first = 0;
         for (size_t i = 0; r == CTLCU_OK && i < sizes.size(); first += sizes[i], ++i) {
@@ -940,8 +944,8 @@ int project_any(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, const d
             if (!r && e == cudaSuccess)
                 e = cudaEventRecord(done, cs);
             if (!r && e == cudaSuccess && threads) {
-                parts.push_back({ d_out + first * view_values, out + first * view_values,
-                                  sizeof(float) * n * view_values, done });
+                parts[n_parts++] = { d_out + first * view_values, out + first * view_values,
+                                     sizeof(float) * n * view_values, done };
                 continue;
             }
             if (!r && e == cudaSuccess)
@@ -954,13 +958,13 @@ int project_any(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, const d
             if (!r && e != cudaSuccess)
                 r = fail(ctx, CTLCU_ERR_CUDA, "copy of projections to the host failed: %s", cudaGetErrorString(e));
         }
-        if (!parts.empty() && r == CTLCU_OK) {
-            const cudaError_t e = ctx->copier.run(ctx->device, parts, true, ctx->copy_stream);
+        if (n_parts && r == CTLCU_OK) {
+            const cudaError_t e = ctx->copier.run(ctx->device, parts, n_parts, true, ctx->copy_stream);
             if (e != cudaSuccess)
-                r = fail(ctx, CTLCU_ERR_CUDA, "copy of projections to the host failed: %s", cudaGetErrorString(e));
+                r = fail(ctx, e == cudaErrorMemoryAllocation ? CTLCU_ERR_OUT_OF_MEMORY : CTLCU_ERR_CUDA, "copy of projections to the host failed: %s", cudaGetErrorString(e));
         }
-        for (HostCopyPart& p : parts)
-            cudaEventDestroy(p.after);
+        for (size_t i = 0; i < n_parts; ++i)
+            cudaEventDestroy(parts[i].after);
         // the device buffers are freed on `st`: order that after the last copy
         // and after everything on the second stream
         cudaEvent_t copied = nullptr, aux_done = nullptr;

@@ -10,7 +10,8 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
-#include <system_error>
+#include <exception>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -56,12 +57,14 @@ struct Piece {
     cudaEvent_t after;  // to wait for, or null
 };
 
-std::vector<Piece> cut(const std::vector<HostCopyPart>& parts)
+std::vector<Piece> cut(const HostCopyPart* parts, size_t n)
 {
     std::vector<Piece> out;
-    for (const HostCopyPart& p : parts)
+    for (size_t i = 0; i < n; ++i) {
+        const HostCopyPart& p = parts[i];
         for (size_t o = 0; o < p.bytes; o += HostCopier::kSlot)
             out.push_back({ (char*)p.device + o, (char*)p.host + o, std::min(HostCopier::kSlot, p.bytes - o), p.after });
+    }
     return out;
 }
 
@@ -114,10 +117,11 @@ cudaError_t work(HostCopier& hc, int device, const std::vector<Piece>& pieces, s
 }  // namespace
 
 // Returns when every byte is in place (to the host) or has left the slots (to the
-// device: the transfers are queued on `st` and done).
-cudaError_t HostCopier::run(int device, const std::vector<HostCopyPart>& parts, bool to_host, cudaStream_t st)
-{
-    const std::vector<Piece> pieces = cut(parts);
+// device: the transfers are queued on `st` and done).  No exception leaves it: it runs
+// behind a C interface.
+cudaError_t HostCopier::run(int device, const HostCopyPart* parts, size_t n_parts, bool to_host, cudaStream_t st)
+try {
+    const std::vector<Piece> pieces = cut(parts, n_parts);
     const int n = (int)std::min<size_t>((size_t)workers, pieces.size());
     std::atomic<size_t> next{ 0 };
     std::vector<cudaError_t> got((size_t)std::max(n, 1), cudaSuccess);
@@ -126,8 +130,8 @@ cudaError_t HostCopier::run(int device, const std::vector<HostCopyPart>& parts, 
     for (int w = 1; w < n; ++w) {
         try {
             threads.emplace_back([&, w] { got[(size_t)w] = work(*this, device, pieces, next, w, to_host, st); });
-        } catch (const std::system_error&) {
-            break;  // the threads there are take the pieces
+        } catch (const std::exception&) {
+            break;  // no thread, or no memory for one: the threads there are take the pieces
         }
     }
     if (n > 0)
@@ -138,6 +142,8 @@ cudaError_t HostCopier::run(int device, const std::vector<HostCopyPart>& parts, 
         if (e != cudaSuccess)
             return e;
     return cudaSuccess;
+} catch (const std::bad_alloc&) {
+    return cudaErrorMemoryAllocation;  // before any thread was started
 }
 
 }  // namespace ctlcu

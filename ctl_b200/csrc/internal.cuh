@@ -385,7 +385,7 @@ struct HostCopier {
     char* slot(int i) { return static_cast<char*>(base) + kSlot * (size_t)i; }
     cudaError_t ensure();
     void release();
-    cudaError_t run(int device, const std::vector<HostCopyPart>& parts, bool to_host, cudaStream_t st);
+    cudaError_t run(int device, const HostCopyPart* parts, size_t n_parts, bool to_host, cudaStream_t st);
 };
 int den_write(const char* path, const void* data, uint32_t elem, uint32_t rows, uint32_t cols, uint32_t count,
               cudaStream_t st, DenStaging* stage, std::string& msg);

@@ -13,8 +13,11 @@
 
 #include <cstdarg>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <map>
+#include <new>
+#include <atomic>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -59,6 +62,8 @@ int capturing = 0, capture_mode = 0, foreign_capture = 0, unsafe_calls = 0;
 int last_mode = 0;
 long next_handle = 16;
 thread_local int current = 0;
+std::atomic<int> news_left{ 0 };            // allocations until the one that fails, counted from
+int news_after_pin = 0;                     // the next pinned allocation on
 std::map<int, uint64_t> free_of_device;     // what cudaMemGetInfo answers there, where set
 
 void note(const char* fmt, ...)
@@ -164,7 +169,27 @@ const char* read(const void* p, cudaStream_t s)
 
 }  // namespace
 
-#define LOCK std::lock_guard<std::mutex> lk_(mu)
+// the library's own allocations
+thread_local int in_fake = 0;
+struct InFake {
+    InFake() { ++in_fake; }
+    ~InFake() { --in_fake; }
+};
+void* operator new(size_t n)
+{
+    if (in_fake == 0 && news_left.load() > 0 && news_left.fetch_sub(1) == 1)
+        throw std::bad_alloc();
+    void* p = malloc(n ? n : 1);
+    if (!p)
+        throw std::bad_alloc();
+    return p;
+}
+void operator delete(void* p) noexcept { free(p); }
+void operator delete(void* p, size_t) noexcept { free(p); }
+
+#define LOCK          \
+    InFake in_fake_;  \
+    std::lock_guard<std::mutex> lk_(mu)
 #define SIM extern "C" __attribute__((visibility("default")))
 
 SIM void sim_reset()
@@ -189,6 +214,8 @@ SIM void sim_capacity(uint64_t bytes) { LOCK; capacity = bytes; }
 SIM uint64_t sim_used() { LOCK; return used; }
 SIM void sim_free_answers(const uint64_t* v, int n) { LOCK; free_answers.assign(v, v + n); }
 SIM void sim_free_of_device(int device, uint64_t bytes) { LOCK; free_of_device[device] = bytes; }
+SIM void sim_fail_new_after_pin(int nth) { LOCK; news_after_pin = nth; }
+SIM void sim_stop_failing_new() { news_left = 0; }
 SIM void sim_fail(const char* what, int nth) { LOCK; failures[what] = nth; }
 SIM void sim_mode_ms(int mode, float ms) { LOCK; mode_ms[mode] = ms; }
 SIM void sim_capturing(int on) { LOCK; capturing = on; }
@@ -372,6 +399,8 @@ cudaError_t cudaHostAlloc(void** p, size_t bytes, unsigned)
     LOCK;
     *p = malloc(bytes);
     pinned[*p] = bytes;
+    news_left = news_after_pin;
+    news_after_pin = 0;
     return cudaSuccess;
 }
 cudaError_t cudaMallocHost(void** p, size_t bytes) { return cudaHostAlloc(p, bytes, 0); }

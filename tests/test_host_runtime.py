@@ -1,5 +1,9 @@
 """What the host side does around its launches, on a simulated CUDA runtime
 (tests/hostsim): the order of streams, and arrays built and freed."""
+import os
+import subprocess
+import sys
+
 import pytest
 
 import hostsim
@@ -215,3 +219,44 @@ def test_memory_that_only_speeds_up_is_given_back_when_it_is_needed(sim, what, h
     sim.clear()
     assert sim.project(a, sim.settings(volume_upsampling=2)) == L.OK
     assert sim.projections()[-1][4] == ("ok" if held else "-")
+
+
+_NO_MEMORY = """
+import sys
+import ctypes as C
+import numpy as np
+import hostsim
+from ctl_b200 import _lib as L
+nth, towards = int(sys.argv[2]), sys.argv[3]
+sim = hostsim.Sim(sys.argv[1])
+data = np.arange(128 ** 3 * 4 // 3, dtype=np.float32)[:128 ** 3].reshape(128, 128, 128)
+v, _ = sim.volume()
+if towards == "device":
+    sim.lib.sim_fail_new_after_pin(nth)
+    h = C.c_uint64()
+    make = lambda: sim.lib.ctlcu_volume_create(sim.h, C.byref(sim.desc((128, 128, 128))), data.ctypes.data, 0, C.byref(h))
+    rc = make()
+    sim.lib.sim_stop_failing_new()
+    assert make() == L.OK
+else:
+    sim.lib.sim_fail_new_after_pin(nth)
+    rc = sim.project(v, sim.settings(), views=9, channels=512, rows=512, host=True)
+    sim.lib.sim_stop_failing_new()
+    assert sim.project(v, sim.settings(), views=9, channels=512, rows=512, host=True) == L.OK
+assert rc in (L.OK, L.ERR_OUT_OF_MEMORY), rc
+print("status", rc)
+"""
+
+
+@pytest.mark.parametrize("towards", ["device", "host"])
+def test_copies_by_threads_do_not_end_the_process_without_host_memory(library, towards):
+    """One allocation of the copying code after another fails (its lists, a thread's start
+    among running threads): the call gives a status, the next one works."""
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([hostsim.ROOT, os.path.dirname(hostsim.HERE)]))
+    statuses = []
+    for nth in range(1, 9):
+        r = subprocess.run([sys.executable, "-c", _NO_MEMORY, library, str(nth), towards], env=env, capture_output=True,
+                           text=True, timeout=120)
+        assert r.returncode == 0, (nth, r.stderr[-400:])
+        statuses.append(int(r.stdout.split()[-1]))
+    assert L.ERR_OUT_OF_MEMORY in statuses
