@@ -63,6 +63,7 @@ struct ctlcu_ctx {
     uint64_t next_handle = 1;
     uint64_t budget = 0;  // 0 = unlimited
     uint64_t used = 0;
+    uint64_t cells_allowed = 0;  // bytes of cells that up-sampled calls may still build without asking
     int* d_flags = nullptr;
     unsigned long long* d_counter = nullptr;
     uint64_t launches = 0;
@@ -309,6 +310,9 @@ void drop_cells(ctlcu_ctx* ctx, VolumeEntry& v)
     else
         cudaFree(v.cells);
     ctx->used -= std::min<uint64_t>(ctx->used, v.cell_bytes);
+    if (v.cells_optional)
+        ctx->cells_allowed += v.cell_bytes;
+    v.cells_optional = false;
     v.cells = nullptr;
     v.cell_bytes = 0;
 }
@@ -441,6 +445,12 @@ int ensure_mean(ctlcu_ctx* ctx, VolumeEntry& v)
     return CTLCU_OK;
 }
 
+size_t cell_array_bytes(const ctlcu_volume_desc& d)
+{
+    const int n[3] = { (int)d.n[0], (int)d.n[1], (int)d.n[2] };
+    return (size_t)cell_layout(n).count * kCellBytes + kSupportBytes;
+}
+
 // Coefficient cells of the padded volume, built once per volume on its first
 // cell-kernel projection, in memory of its own or (`pooled`) of the stream-ordered pool.
 int ensure_cells(ctlcu_ctx* ctx, VolumeEntry& v, bool pooled)
@@ -449,7 +459,7 @@ int ensure_cells(ctlcu_ctx* ctx, VolumeEntry& v, bool pooled)
         return CTLCU_OK;
     const int n[3] = { (int)v.desc.n[0], (int)v.desc.n[1], (int)v.desc.n[2] };
     const CellLayout L = cell_layout(n);
-    const size_t bytes = (size_t)L.count * kCellBytes + kSupportBytes;
+    const size_t bytes = cell_array_bytes(v.desc);
     if (ctx->budget && ctx->used + bytes > ctx->budget)
         return fail(ctx, CTLCU_ERR_OUT_OF_MEMORY,
                     "cell array of %zu bytes exceeds the memory budget (%llu of %llu bytes used)", bytes,
@@ -556,14 +566,21 @@ int ensure_texture(ctlcu_ctx* ctx, VolumeEntry& v, int f, cudaTextureObject_t* o
     return CTLCU_OK;
 }
 
-// Whether the current device has the room for the cells of `times` such volumes that
-// up-sampled calls build: a quarter of its free memory.
-bool room_for_cells(const ctlcu_volume_desc& d, uint32_t times)
+// Whether the context's device has the room for the cells of `times` such volumes that
+// up-sampled calls build: what the context still allows itself, or a quarter of the free
+// memory, asked for anew.  Asking takes 0.1 ms, and on a busy host up to 90 (37^3, 10
+// views of 79 x 73: 0.20 ms in the gather loop, 0.4 to 1 with a question for every new
+// volume, 0.09 without).
+bool room_for_cells(ctlcu_ctx* ctx, const ctlcu_volume_desc& d, uint32_t times)
 {
-    const int n[3] = { (int)d.n[0], (int)d.n[1], (int)d.n[2] };
-    size_t free_bytes = 0, total = 0;
-    if (cudaMemGetInfo(&free_bytes, &total) == cudaSuccess && cell_layout(n).count * kCellBytes * times <= free_bytes / 4)
+    const uint64_t bytes = (uint64_t)cell_array_bytes(d) * times;
+    if (bytes <= ctx->cells_allowed)
         return true;
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) == cudaSuccess && bytes <= free_bytes / 4) {
+        ctx->cells_allowed = free_bytes / 4;
+        return true;
+    }
     cudaGetLastError();
     return false;
 }
@@ -571,7 +588,7 @@ bool room_for_cells(const ctlcu_volume_desc& d, uint32_t times)
 // Whether an up-sampled projection reads the coefficient cells: they are built
 // already, or this call may build them.  The gather loop serves such calls without
 // any array, so one is built only where nothing else can miss the memory: no
-// budget set, at most a quarter of the free device memory, and not while the
+// budget set, room for it (room_for_cells), and not while the
 // context's stream is being captured (an allocation would end the capture).  The memory
 // is the pool's, so that the first call on a new volume costs less than in the gather
 // loop (volume, one pose and release, ms: 64^3 -> 64^2 0.35 in the gather loop, 0.90 with
@@ -583,10 +600,11 @@ bool cells_for_upsampling(ctlcu_ctx* ctx, VolumeEntry& v, bool may_build)
         return false;
     if (v.cells)
         return true;
-    if (!may_build || ctx->budget || is_capturing(ctx->stream) || (v.up == UpLoop::Ask && !room_for_cells(v.desc, 1)))
+    if (!may_build || ctx->budget || is_capturing(ctx->stream) || (v.up == UpLoop::Ask && !room_for_cells(ctx, v.desc, 1)))
         return false;
     if (ensure_cells(ctx, v, true) == CTLCU_OK) {
         v.cells_optional = true;
+        ctx->cells_allowed -= std::min<uint64_t>(ctx->cells_allowed, v.cell_bytes);
         return true;
     }
     cudaGetLastError();
@@ -1458,7 +1476,7 @@ bool ctlcu::upsampled_reads_cells(ctlcu_ctx* ctx, const ctlcu_volume_desc* desc,
 {
     std::lock_guard<std::mutex> lk(ctx->mu);
     cudaSetDevice(ctx->device);
-    return !ctx->budget && room_for_cells(*desc, times);
+    return !ctx->budget && room_for_cells(ctx, *desc, times);
 }
 
 extern "C" {
@@ -1515,6 +1533,11 @@ int ctlcu_create(int device, ctlcu_ctx** out)
         delete ctx;
         return CTLCU_ERR_CUDA;
     }
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) == cudaSuccess)
+        ctx->cells_allowed = free_bytes / 8;
+    else
+        cudaGetLastError();
     *out = ctx;
     return CTLCU_OK;
 }

@@ -37,7 +37,7 @@ def build(folder: str) -> str:
 class Sim:
     """One context of the simulated library."""
 
-    def __init__(self, path: str):
+    def __init__(self, path: str, free_at_creation: int = 0):
         self.lib = lib = C.CDLL(path)
         for name, res, args in L.SIGNATURES:
             fn = getattr(lib, name, None)  # the geometry encoder is not built
@@ -52,6 +52,7 @@ class Sim:
         lib.sim_mode_ms.argtypes = [C.c_int, C.c_float]
         lib.sim_free_of_device.argtypes = [C.c_int, C.c_uint64]
         lib.sim_reset()
+        self.free_answers([free_at_creation])
         self.h = C.c_void_p()
         assert lib.ctlcu_create(0, C.byref(self.h)) == L.OK
 

@@ -59,7 +59,7 @@ std::vector<uint64_t> free_answers;         // what cudaMemGetInfo answers next
 std::string record;
 uint64_t capacity = 180ull << 30, used = 0;
 int capturing = 0, capture_mode = 0, foreign_capture = 0, unsafe_calls = 0;
-int last_mode = 0;
+int last_mode = 0, info_calls = 0;
 long next_handle = 16;
 thread_local int current = 0;
 std::atomic<int> news_left{ 0 };            // allocations until the one that fails, counted from
@@ -220,6 +220,7 @@ SIM void sim_fail(const char* what, int nth) { LOCK; failures[what] = nth; }
 SIM void sim_mode_ms(int mode, float ms) { LOCK; mode_ms[mode] = ms; }
 SIM void sim_capturing(int on) { LOCK; capturing = on; }
 SIM void sim_foreign_capture(int on) { LOCK; foreign_capture = on; unsafe_calls = 0; }
+SIM int sim_info_calls() { LOCK; return info_calls; }
 SIM int sim_unsafe_calls() { LOCK; return unsafe_calls; }
 SIM void* sim_device_memory(uint64_t bytes)
 {
@@ -414,6 +415,7 @@ cudaError_t cudaFreeHost(void* p)
 cudaError_t cudaMemGetInfo(size_t* f, size_t* t)
 {
     LOCK;
+    ++info_calls;
     *t = capacity;
     *f = used < capacity ? capacity - used : 0;
     if (free_of_device.count(current))

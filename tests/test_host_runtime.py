@@ -168,7 +168,7 @@ def test_a_batch_too_large_with_a_lane_per_sub_ray_goes_without(sim, form, reque
 def test_a_group_projects_all_its_views_with_one_loop(sim, devices, free, loop, views):
     """Whether an up-sampled volume's cells are built goes by the free memory, which
     differs from device to device: the group decides once for all its devices, as the
-    result has to be a one-device call's bit for bit.  (A 16^3 volume's cells take 277
+    result has to be a one-device call's bit for bit.  (A 16^3 volume's cells take 231
     KB, a quarter of 1.6 MB holds one context's and not two.)"""
     import ctypes as C
     import numpy as np
@@ -218,7 +218,8 @@ def test_memory_that_only_speeds_up_is_given_back_when_it_is_needed(sim, what, h
     assert sim.memory_used() == used if held else sim.memory_used() != used
     sim.clear()
     assert sim.project(a, sim.settings(volume_upsampling=2)) == L.OK
-    assert sim.projections()[-1][4] == ("ok" if held else "-")
+    # (a result in host memory has left the device again)
+    assert sim.projections()[-1][4] == ("ok" if held or what == "result" else "-")
 
 
 _NO_MEMORY = """
@@ -260,3 +261,30 @@ def test_copies_by_threads_do_not_end_the_process_without_host_memory(library, t
         assert r.returncode == 0, (nth, r.stderr[-400:])
         statuses.append(int(r.stdout.split()[-1]))
     assert L.ERR_OUT_OF_MEMORY in statuses
+
+
+def test_new_volumes_do_not_ask_for_the_free_memory(library):
+    """cudaMemGetInfo can take longer than a small projection: a context asks when it is
+    made, and again only when up-sampled calls have built more cells than that allows.
+    What is freed is allowed again."""
+    s = hostsim.Sim(library, free_at_creation=6 * 1000000)  # an eighth: three 16^3 volumes' cells of 231 KB
+    try:
+        before = s.lib.sim_info_calls()
+        for _ in range(20):
+            v, _ = s.volume()
+            s.clear()
+            assert s.project(v, s.settings(volume_upsampling=2)) == L.OK
+            assert {p[0] for p in s.projections()} == {hostsim.SEGMENTS_UP}
+            assert s.lib.ctlcu_volume_release(s.h, v) == L.OK
+        assert s.lib.sim_info_calls() == before
+        loops = []
+        s.free_answers([1000, 1200000])  # the fourth volume's look, and the fifth's
+        for _ in range(5):
+            v, _ = s.volume()
+            s.clear()
+            assert s.project(v, s.settings(volume_upsampling=2)) == L.OK
+            loops += [p[0] for p in s.projections()]
+        assert loops == [hostsim.SEGMENTS_UP] * 3 + [hostsim.GATHER, hostsim.SEGMENTS_UP]
+        assert s.lib.sim_info_calls() == before + 2
+    finally:
+        s.close()
