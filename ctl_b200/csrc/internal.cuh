@@ -366,7 +366,7 @@ struct DenStaging {
 };
 // Copies between pageable host memory and the device by several threads through pinned
 // slots (hostcopy.cu); a context keeps one, allocated on first use: at most 8 threads'
-// slots, 32 MB.
+// slots, 16 MB.
 struct HostCopyPart {
     void* device;
     void* host;         // read only when copying to the device
@@ -374,7 +374,10 @@ struct HostCopyPart {
     cudaEvent_t after;  // event the copy waits for, or null
 };
 struct HostCopier {
-    static constexpr size_t kSlot = 2u << 20;
+    // Pinning the slots takes as long as a first call saves: 256^3 from the host, 30 x 512^2
+    // back, first / later calls of a context, ms: 512 KB 25 / 8.7, 1 MB 29 / 7.9, 2 MB 39 /
+    // 7.9; with the driver's copies 29 / 16.8
+    static constexpr size_t kSlot = 1u << 20;
     static constexpr int kMaxWorkers = 8;
     // from here on the threads' start costs less than they save
     static constexpr size_t kLeast = 8u << 20;
