@@ -213,6 +213,7 @@ class DRRServer:
         self.budget = self._free_budget()
         used = 0
         done = refused = batches = batched = 0
+        turn = 0  # the stream that a new batch tries first
         torch.cuda.synchronize()
         base = torch.cuda.Event(enable_timing=True)
         base.record(self.streams[0])
@@ -234,8 +235,12 @@ class DRRServer:
                 pending.pop()
                 used += need
                 queue.append(r)
-            # completions, then new batches on free streams
-            for i, s in enumerate(self.streams):
+            # completions, then new batches on free streams, the streams in turn: results
+            # come from their stream's share of the reserved memory, and with short
+            # requests the first stream would be free for nearly all of them and use up
+            # its share while the others' is idle
+            for i in [(turn + k) % len(self.streams) for k in range(len(self.streams))]:
+                s = self.streams[i]
                 slot = inflight[i]
                 if slot is not None and slot[1].query():
                     ms = base.elapsed_time(slot[1])
@@ -285,6 +290,7 @@ class DRRServer:
                         ev = torch.cuda.Event(enable_timing=True)
                         ev.record(s)
                     inflight[i] = (batch, ev)
+                    turn = (i + 1) % len(self.streams)
                     batches += 1
                     batched += len(batch)
         wall = time.perf_counter() - t0

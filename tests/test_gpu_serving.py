@@ -129,3 +129,27 @@ def test_reserved_server_allocates_nothing_while_serving():
     del reqs
     h.release()
     ctx.close()
+
+
+def test_short_requests_take_the_streams_in_turn():
+    """Requests that are done before the next one arrives: their results, 100 blocks of 1 MB
+    held by the requests, come from all four streams' shares of 32 MB, not from one."""
+    import torch
+    ctx = Context(0)
+    vol = Ph.ellipsoid_phantom((32, 32, 32), (3, 3, 3), 4, seed=13)
+    h = ctx.volume(VoxelVolume(vol, (3, 3, 3)))
+    server = DRRServer(ctx, [h], 48, 40, Settings(), streams=4, max_batch=1, reserve_bytes=128 << 20)
+    server.warm_up()
+    reqs = poisson_requests(20000.0, 100, 1, _base_view(), seed=17, views=(1, 2))
+    for i, r in enumerate(reqs):
+        r.arrival = 0.002 * i
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_stats().get("segment.all.allocated", 0)
+    stats = server.run(reqs)
+    assert stats.completed == 100
+    assert torch.cuda.memory_stats().get("segment.all.allocated", 0) == before
+    alone = ctx.project(h, reqs[50].pmats, 48, 40, Settings())
+    np.testing.assert_array_equal(reqs[50].out.cpu().numpy(), alone)
+    del reqs
+    h.release()
+    ctx.close()
