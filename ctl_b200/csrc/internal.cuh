@@ -190,7 +190,17 @@ inline PairLayout pair_layout(const int n[3])
     return L;
 }
 
-enum class Mode : int { Trilinear = 0, Nearest = 1, Texture = 2, Cells = 3, Pairs = 4, Segments = 5, CellsUp = 6, SegmentsUp = 7, NearestSamples = 8 };
+enum class Mode : int {
+    Trilinear = 0,
+    Nearest = 1,
+    Texture = 2,
+    Cells = 3,
+    Pairs = 4,
+    Segments = 5,
+    CellsUp = 6,
+    SegmentsUp = 7,
+    NearestSamples = 8
+};
 enum class Accum : int { F64 = 0, Kahan = 1, F32 = 2 };
 
 // Everything a projection launch needs, passed by value.
@@ -256,8 +266,9 @@ struct BatchReq {
 // Up to this ray_sampling the cells are read segment by segment, above it sample
 // by sample.  A segment costs about twice a sample, so it pays while it holds two
 // samples or so.  Segments / samples, ms, at ray_sampling 0.3, 0.5, 0.6, 0.75, 1:
-//   201x173x155 -> 23 x 479x361      2.00 / 2.99, 1.89 / 2.16, 1.83 / 1.92, 1.75 / 1.65, 1.55 / 1.33
-//   512^3 helical, 180 x 64 x 16^2   2.16 / 3.58, 2.05 / 2.75, 1.99 / 2.53, 1.90 / 2.25, 1.73 / 1.97
+//   201x173x155 -> 23 x 479x361      1.38 / 2.12, 1.30 / 1.50, 1.27 / 1.32, 1.21 / 1.13, 1.09 / 0.90
+//   512^3 helical, 180 x 64 x 16^2   1.54 / 2.56, 1.48 / 1.91, 1.44 / 1.75, 1.38 / 1.54, 1.26 / 1.32
+//   256^3 -> 30 x 512^2              4.53 / 7.37, 4.33 / 5.17, 4.16 / 4.49, 3.98 / 3.73, 3.46 / 2.86
 // The rule looks at the setting alone, so that a request takes the same loop in a
 // batch as on its own.
 constexpr float kSegmentMaxSampling = 0.6f;

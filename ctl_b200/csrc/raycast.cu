@@ -188,8 +188,8 @@ __device__ __forceinline__ Ray setup_ray(const ProjectArgs& a, const ViewGeom& g
 // the face tests above let in and that is not zero.  Lengths are in grid voxels from
 // the box's low corner; the host's scale, inv_voxel and corner_v leave one reciprocal
 // square root and three reciprocals of the 18 divisions above (64^3 -> 90 x 128^2:
-// 311 -> 299 us; 201x173x155 -> 23 x 479 x 361: 2.03 -> 1.95 ms).  Coordinates are v = p - 1 + pad: the cell index is rint(v), the offset
-// from the cell centre v - rint(v).
+// 311 -> 299 us; 201x173x155 -> 23 x 479 x 361: 2.03 -> 1.95 ms).  Coordinates are
+// v = p - 1 + pad: the cell index is rint(v), the offset from the cell centre v - rint(v).
 template <Mode M>
 __device__ __forceinline__ Ray setup_ray_cells(const ProjectArgs& a, const ViewGeom& g, double px, double py,
                                                int* flags)
@@ -592,7 +592,8 @@ __device__ __forceinline__ void cell_segment(const char* __restrict__ cells, flo
 
 // Samples per window of the segment loop: the lanes of a warp, which step from
 // cell to cell each at its own pace, meet again at every sample index that is a
-// multiple of this, where positions are also formed anew (advance_axis).  Without that they drift apart by several cells along a long
+// multiple of this, where positions are also formed anew (advance_axis).  Without that
+// they drift apart by several cells along a long
 // ray, share fewer cells per load and conflict more in L1 (256^3 -> 60 x 512^2
 // with windows of 128, 192 and 256 samples: 11.48, 11.26 and 11.39 ms; 512^3
 // helical, 180 views: 2.18, 2.17 and 2.19 ms.  Before positions were formed anew at
