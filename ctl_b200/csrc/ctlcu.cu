@@ -600,7 +600,8 @@ bool cells_for_upsampling(ctlcu_ctx* ctx, VolumeEntry& v, bool may_build)
         return false;
     if (v.cells)
         return true;
-    if (!may_build || ctx->budget || is_capturing(ctx->stream) || (v.up == UpLoop::Ask && !room_for_cells(ctx, v.desc, 1)))
+    if (!may_build || ctx->budget || is_capturing(ctx->stream) ||
+        (v.up == UpLoop::Ask && !room_for_cells(ctx, v.desc, 1)))
         return false;
     if (ensure_cells(ctx, v, true) == CTLCU_OK) {
         v.cells_optional = true;
@@ -979,7 +980,8 @@ int project_any(ctlcu_ctx* ctx, VolumeEntry& v, const ctlcu_settings* s, const d
         if (n_parts && r == CTLCU_OK) {
             const cudaError_t e = ctx->copier.run(ctx->device, parts, n_parts, true, ctx->copy_stream);
             if (e != cudaSuccess)
-                r = fail(ctx, e == cudaErrorMemoryAllocation ? CTLCU_ERR_OUT_OF_MEMORY : CTLCU_ERR_CUDA, "copy of projections to the host failed: %s", cudaGetErrorString(e));
+                r = fail(ctx, e == cudaErrorMemoryAllocation ? CTLCU_ERR_OUT_OF_MEMORY : CTLCU_ERR_CUDA,
+                         "copy of projections to the host failed: %s", cudaGetErrorString(e));
         }
         for (size_t i = 0; i < n_parts; ++i)
             cudaEventDestroy(parts[i].after);
@@ -1195,8 +1197,8 @@ int prepare_batch(ctlcu_ctx* ctx, const ctlcu_request* requests, uint32_t n, con
     bp.shape = shape_of(&eff);
     // all work items in 31 bits, and the persistent launch's warps in 32 with room for the
     // counter to run past; a lane for every sub-ray only where that holds
-    const uint64_t most = persistent ? std::min<uint64_t>(0x7fffffffull, (0xffffffffull - (1ull << 20)) / (bp.shape.block / 32))
-                                     : 0x7fffffffull;
+    const uint64_t warps = bp.shape.block / 32, counted = (0xffffffffull - (1ull << 20)) / warps;
+    const uint64_t most = persistent ? std::min<uint64_t>(0x7fffffffull, counted) : 0x7fffffffull;
     uint64_t spread_items = 0;
     for (uint32_t i = 0; i < n; ++i) {
         ProjectArgs a = {};

@@ -68,7 +68,9 @@ typedef enum {
  * Sample-loop variant.  AUTO picks CELLS for software trilinear interpolation
  * without up-sampling and GATHER otherwise; with up-sampling (>= 2) it reads the
  * cell array in place of the voxels where that array exists or a context without
- * a memory budget has the room for it.
+ * a memory budget has the room for it (one or the other for all views of a call; the
+ * two agree to FP32 rounding).  An array built for that is freed when a volume, a
+ * result or another loop's array needs the memory.
  *   GATHER  eight scalar loads per sample from the zero-padded voxel array
  *   CELLS   32-byte loads from a derived cell array holding, per trilinear cell,
  *           the 8 coefficients of its interpolation polynomial about the cell
